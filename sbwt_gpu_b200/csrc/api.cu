@@ -326,7 +326,7 @@ extern "C" void sbwt_index_free(sbwt_index *ix) {
     cudaFree(ix->d_scan);
     cudaFree(ix->d_node);
     cudaFree(ix->d_sel);
-    cudaFree(ix->d_back);
+    sbwt::free_walk(ix);
     for (int i = 0; i < sbwt_index::kPipeSlots; i++) {
         ix->ws[i].release();
         if (ix->pipe_stream[i]) cudaStreamDestroy(ix->pipe_stream[i]);
@@ -536,13 +536,11 @@ void l2_setaside_release(sbwt_index *ix) {
 void set_gather_policies(const sbwt_index *ix, SearchArgs &a) {
     const u64 half = ix->l2_bytes / 2;
     const u64 pre_bytes = ix->p ? (1ull << (2 * ix->p)) * (ix->pre64 ? 16ull : 8ull) : 0;
-    const u64 back_bytes = ix->d_back ? ix->n * 8ull : 0;
     const int ev = ix->shape.evict;
     a.ef_pre = a.runs && ev != 1 && (ev == 2 || pre_bytes > half);
-    a.ef_back = a.runs && ev != 1 && (ev == 2 || back_bytes > half);
 }
 
-SearchArgs base_args(const sbwt_index *ix, bool rows) {
+SearchArgs base_args(const sbwt_index *ix, bool rows, u64 n_kmers, bool filtered) {
     SearchArgs a;
     std::memset(&a, 0, sizeof(a));
     a.lines = ix->d_lines;
@@ -559,10 +557,15 @@ SearchArgs base_args(const sbwt_index *ix, bool rows) {
     a.k = ix->k;
     a.chunk = search_chunk(ix, rows);
     a.runs = rows && runs_form(ix);
-    a.stream = a.runs && stream_form(ix);
+    a.stream = a.runs && filtered && stream_form(ix);
+    a.walk = a.runs && !filtered && stream_form(ix);
     a.index64 = (u32)ix->shape.index64;
     a.pre32 = a.runs ? ix->d_pre32 : nullptr;
-    if (a.stream) a.sv = stream_view(ix);
+    if (a.stream || a.walk) a.sv = stream_view(ix);
+    if (a.walk) {
+        a.wv = walk_view(ix);
+        a.chunk = walk_chunk(ix, n_kmers);
+    }
     set_gather_policies(ix, a);
     return a;
 }
@@ -575,7 +578,7 @@ int search_rows_device(sbwt_index *ix, Workspace &w, const uint8_t *d_letters, u
                        u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s) {
     if (n_rows == 0 || n_kmers == 0) return 0;
     const u64 n_words = (n_letters + 32 + 31) / 32;
-    SearchArgs a = base_args(ix, true);
+    SearchArgs a = base_args(ix, true, n_kmers);
     if (!d_answers && !a.runs) {  // membership only: the per-k-mer kernels derive it from answers
         SBWT_TRY(grow(w.answers, w.answers_cap, n_kmers));
         d_answers = w.answers;
@@ -703,7 +706,7 @@ extern "C" int sbwt_search_packed(sbwt_index *ix, const uint64_t *d_kmer_string,
     if (runs_form(ix)) {
         // runs of consecutive positions go to the run-walking kernel (packed_runs.cu); the run
         // count stays on the device, and of the two launches below only the one it chose searches
-        SearchArgs a = base_args(ix, true);
+        SearchArgs a = base_args(ix, true, n_kmers);
         SBWT_TRY(packed_runs(w, d_positions_in_results_out, n_kmers, a.chunk, s, &runs_dev));
         a.words = d_kmer_string;
         a.positions = nullptr;
@@ -718,7 +721,7 @@ extern "C" int sbwt_search_packed(sbwt_index *ix, const uint64_t *d_kmer_string,
         a.counter = w.counter;
         SBWT_TRY(launch_search(ix, a, s, nullptr));
     }
-    SearchArgs a = base_args(ix, false);
+    SearchArgs a = base_args(ix, false, n_kmers);
     a.words = d_kmer_string;
     a.positions = d_positions_in_results_out;
     a.runs_dev = runs_dev;

@@ -44,12 +44,15 @@ struct SearchArgs {
     u64 n_kmers;
     unsigned long long *counter;  // work-stealing cursor (zeroed before launch)
     u32 chunk;                    // k-mers per grab; with `runs`, k-mers per window of chunk_row
+    u32 piece;                    // with `walk`: k-mers per run at most
     u32 runs;                     // read mode: walk runs right to left with the absent-run skip
     u32 stream;                   // with `runs`: backward steps from a found k-mer (needs sv)
     u32 index64;                  // with `runs`: the walk's 64-bit index form whatever the batch size
-    u32 ef_pre, ef_back;          // with `runs`: evict-first gathers from the presearch / backward
-                                  // table (each set when that table cannot stay in L2; device.cuh)
-    dev::StreamView sv;           // backward table, node nibbles, select samples (stream.cuh)
+    u32 ef_pre;                   // with `runs`: evict-first gathers from the presearch table (set when
+                                  // it cannot stay in L2; device.cuh)
+    u32 walk;                     // read mode: the forward walk (walk.cu), with wv and sv
+    dev::StreamView sv;           // node nibbles, select samples (stream.cuh)
+    dev::WalkView wv;             // labels, q-mer bitmap, group marks (stream.cuh)
     uint32_t *member;             // with `runs`: membership bitmap written by the search kernel, or NULL
     // k-mer list mode: k-mer j is kmer_list[j] (MSB-first word)
     const u64 *kmer_list;
@@ -145,10 +148,14 @@ struct sbwt_index {
     uint32_t *d_pre32 = nullptr;
     bool pre64 = false;
     int compact_pre = -1;  // the compact table: -1 = from SBWT_PRESEARCH_COMPACT, 0 = off, 1 = on
-    // backward-step structures (stream.cu): node nibbles, select samples, backward table
+    // backward-step structures (stream.cu): node nibbles, select samples
     uint8_t *d_node = nullptr;
     uint32_t *d_sel = nullptr;
-    uint64_t *d_back = nullptr;  // backward table (stream.cuh, SBWT_BACK_TABLE)
+    // structures of the forward walk (WalkView, stream.cuh); walk_q = 0: not there
+    uint64_t *d_labels = nullptr;
+    uint32_t *d_qbits = nullptr, *d_marks = nullptr, *d_path_node = nullptr, *d_node_pos = nullptr;
+    ulonglong2 *d_path = nullptr;
+    uint32_t walk_q = 0;
     uint32_t sel_off[4] = {0, 0, 0, 0}, sel_n[4] = {0, 0, 0, 0};
     bool stream_ok = false;
     // device ms of the last build of: lines, poppy, presearch table, backward-step structures
@@ -212,6 +219,8 @@ int launch_kmer_list(const SearchArgs &a, uint64_t j0, uint64_t count, uint64_t 
 // stream.cu
 int build_stream(sbwt_index *ix, cudaStream_t s);
 dev::StreamView stream_view(const sbwt_index *ix);
+void free_walk(sbwt_index *ix);
+dev::WalkView walk_view(const sbwt_index *ix);
 
 // packed_runs.cu
 // The kernel contract's runs are walked when they average at least
@@ -223,7 +232,8 @@ int packed_runs(Workspace &w, const u64 *positions, u64 n_kmers, u32 chunk, cuda
 // api.cu
 // Launch arguments of a search with the index's current shape and mode (the
 // batch pointers left NULL); `rows`: a batch of reads.
-SearchArgs base_args(const sbwt_index *ix, bool rows);
+// `filtered`: behind the learned prefilter (the run walk, never the forward walk).
+SearchArgs base_args(const sbwt_index *ix, bool rows, u64 n_kmers, bool filtered = false);
 // Grows w for a batch of reads and enqueues pack -> per-row k-mer table ->
 // chunk table on s; fills the batch fields of a (a.chunk set by base_args).
 int prepare_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_letters, uint64_t n_letters,
@@ -255,5 +265,10 @@ bool stream_form(const sbwt_index *ix);
 // k-mers per window of the row table.  `rows`: a batch of reads.
 u32 search_chunk(const sbwt_index *ix, bool rows);
 bool search_shape_supported(const KernelShape &sh, bool wide);
+bool run32_ok(const SearchArgs &a);
+
+// walk.cu
+u32 walk_chunk(const sbwt_index *ix, u64 n_kmers);
+int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *launched_blocks);
 
 }  // namespace sbwt

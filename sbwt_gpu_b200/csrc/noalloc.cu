@@ -74,7 +74,7 @@ extern "C" int sbwt_search_reads_noalloc(sbwt_index *ix, const uint8_t *d_letter
     if (!d_answers && !d_member_bits) return set_error("NULL answers and membership pointers");
     SBWT_CHECK_CUDA(cudaSetDevice(ix->device));
     const cudaStream_t s = (cudaStream_t)stream;
-    SearchArgs a = base_args(ix, true);
+    SearchArgs a = base_args(ix, true, n_kmers);
     // membership only: the run-walking kernel writes the bitmap itself; the
     // per-k-mer kernels derive it from answers, which then go to the scratch
     const bool scratch_answers = !d_answers && !a.runs;

@@ -208,7 +208,7 @@ int search_list(sbwt_index *ix, const uint64_t *d_kmers, uint64_t n, uint64_t *d
     if (n == 0) return 0;
     Workspace &w = ix->ws[0];
     SBWT_TRY(grow(w.counter, w.counter_cap, 1));
-    SearchArgs a = base_args(ix, false);
+    SearchArgs a = base_args(ix, false, n);
     a.kmer_list = d_kmers;
     a.answers = d_answers;
     a.n_kmers = n;
@@ -539,7 +539,7 @@ extern "C" int sbwt_search_reads_filtered(sbwt_index *ix, sbwt_prefilter *pf, co
     SBWT_CHECK_CUDA(cudaSetDevice(ix->device));
     cudaStream_t s = (cudaStream_t)stream;
     Workspace &w = ix->ws[0];
-    SearchArgs a = base_args(ix, true);
+    SearchArgs a = base_args(ix, true, n_kmers, true);
     if (!a.runs || ix->shape.layout != SBWT_LAYOUT_LINES)
         return set_error("the prefiltered search of reads needs the run walk on the line layout "
                          "(search mode stream or skip, one lane per k-mer, queue-fed)");

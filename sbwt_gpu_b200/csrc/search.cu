@@ -28,6 +28,7 @@
 
 #include "device.cuh"
 #include "internal.h"
+#include "launch.cuh"
 #include "mlp_kernels.cuh"
 #include "rank.cuh"
 
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(128, RunsMinBlocks<R, IX>::value) search_runs_
             if (STREAM && V != dev::kNoNode) {
                 // ---- backward step: k-mer J = x[J] . (first k-1 letters of k-mer J+1)
                 const u32 letter = (u32)(a.words[pos >> 5] >> (62u - 2u * (u32)(pos & 31u))) & 3u;
-                const u32 u = a.sv.back_step(V, letter, a.ef_back, l2_evict_first_policy());
+                const u32 u = a.sv.back_step(V, letter);
                 adv = 1;
                 if (u != dev::kNoNode) found = u;
             } else if (FILTER && ((__ldg(a.reject + (J >> 5)) >> (J & 31u)) & 1u)) {
@@ -711,27 +712,6 @@ __global__ void __launch_bounds__(128, RunsMinBlocks<R, IX>::value) search_runs_
 
 // -------------------------------------------------------------- dispatch
 
-// Launches a search kernel with the L2 access-policy window of the index's
-// rank lines, where one applies (l2_window).
-template <class K, class R>
-int launch_kernel(K kern, u32 blocks, u32 threads, cudaStream_t s, const sbwt_index *ix, const R &rk,
-                  const SearchArgs &a) {
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cfg.numAttrs = 0;
-    if (l2_window(ix, &attr[0].val.accessPolicyWindow)) {
-        attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    SBWT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, rk, a));
-    return 0;
-}
-
 template <class R, int KPT, int TPK>
 int launch_one(const R &rk, SearchArgs &a, const sbwt_index *ix, cudaStream_t s, u32 tpb, u32 *blocks_out) {
     auto kern = search_kernel<R, KPT, TPK>;
@@ -745,23 +725,13 @@ int launch_one(const R &rk, SearchArgs &a, const sbwt_index *ix, cudaStream_t s,
     return 0;
 }
 
-// The batch fits the 32-bit form of the walk: every k-mer index, letter
-// offset and row index with a window's slack below 2^32 (a letter offset
-// read from a bad row table is still clamped to max_pos).  SBWT_RUN_INDEX64=1
-// in the environment when an index is created keeps its walks on the 64-bit
-// form.
-bool run32_ok(const SearchArgs &a) {
-    const u64 lim = (1ull << 32) - (1ull << 16);
-    return !a.index64 && a.n_kmers < lim && a.max_pos < lim && a.n_rows < lim;
-}
-
 template <class R, u32 WIN, class IX>
 auto runs_kernel_ix(const SearchArgs &a) {
     if constexpr (std::is_same<R, LinesRankerT<1>>::value) {  // the prefiltered walk: line layout only
         if (a.reject)
             return a.stream ? search_runs_kernel<R, true, true, WIN, IX> : search_runs_kernel<R, false, true, WIN, IX>;
     }
-    return a.stream ? search_runs_kernel<R, true, false, WIN, IX> : search_runs_kernel<R, false, false, WIN, IX>;
+    return search_runs_kernel<R, false, false, WIN, IX>;
 }
 
 template <class R, u32 WIN>
@@ -848,6 +818,16 @@ int poppy_sb(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, const KernelSh
 
 }  // namespace
 
+// The batch fits the 32-bit form of the walk: every k-mer index, letter
+// offset and row index with a window's slack below 2^32 (a letter offset
+// read from a bad row table is still clamped to max_pos).  SBWT_RUN_INDEX64=1
+// in the environment when an index is created keeps its walks on the 64-bit
+// form.
+bool run32_ok(const SearchArgs &a) {
+    const u64 lim = (1ull << 32) - (1ull << 16);
+    return !a.index64 && a.n_kmers < lim && a.max_pos < lim && a.n_rows < lim;
+}
+
 bool runs_form(const sbwt_index *ix) {
     const KernelShape &sh = ix->shape;
     if (sh.mode == SBWT_SEARCH_EVERY_KMER || sh.kpt != 0) return false;
@@ -858,7 +838,7 @@ bool runs_form(const sbwt_index *ix) {
 }
 
 bool stream_form(const sbwt_index *ix) {
-    return runs_form(ix) && ix->shape.mode == SBWT_SEARCH_STREAM && ix->stream_ok;
+    return runs_form(ix) && ix->shape.mode == SBWT_SEARCH_STREAM && ix->stream_ok && ix->walk_q;
 }
 
 u32 search_chunk(const sbwt_index *ix, bool rows) {
@@ -872,6 +852,7 @@ u32 search_chunk(const sbwt_index *ix, bool rows) {
 int launch_search(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *blocks) {
     const KernelShape &sh = ix->shape;
     if (a.n_kmers == 0) return 0;
+    if (a.walk) return launch_walk(ix, a, s, blocks);
     if (a.reject && !(a.runs && sh.layout == SBWT_LAYOUT_LINES && sh.tpk == 1 && sh.kpt == 0))
         return set_error("the prefiltered search of reads needs the run walk on the line layout "
                          "(search mode stream or skip, one lane per k-mer, queue-fed)");

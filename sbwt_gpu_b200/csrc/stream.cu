@@ -6,14 +6,16 @@
 // First letters and groups come from the labels: with pred(v) = the first
 // node of the group of v's predecessor (stream.cuh), the last letter of
 // pred^t(v) is label(v)[k-1-t] for t < k, and the chain reaches the all-$
-// root exactly where the label's $ padding starts.  Pointer doubling builds,
-// for every node, the last min(32, real letters) letters of its label in
-// five rounds of gathers:
+// root exactly where the label's $ padding starts.  Labels roll along the paths
+// (write_segment) into
 //   code(v) = sum_t lastletter(pred^t(v)) << 2t,  len(v) = letters before the root
 // Then first letter = letter k-1 (or $ if len < k), and v starts a group iff
 // its last k-1 letters (and how many of them are real) differ from v-1's.
+#include <algorithm>
 #include <cstring>
 #include <vector>
+
+#include <cub/cub.cuh>
 
 #include "internal.h"
 #include "stream.cuh"
@@ -36,43 +38,135 @@ __global__ void select_samples_kernel(const ulonglong4 *__restrict__ lines, u32 
     for (u32 s = s_lo; s <= s_hi && s < n_samples; s++) sel[s] = t;
 }
 
-__global__ void pred_init_kernel(const StreamView sv, u32 *__restrict__ P, u64 *__restrict__ code,
-                                 uint8_t *__restrict__ len, unsigned long long *__restrict__ bad) {
+// ---- paths: each column's first outgoing edge links it to one successor, and
+// every node but the root has one incoming edge, so the links form chains and
+// cycles.  They are cut into segments at the nodes without a link to them and at
+// one node in kSegment (by a hash), so that one thread per segment walks it: once
+// to size it, once to write it together with the labels, which roll along the
+// segment from its first node's (k select steps back).
+
+constexpr u32 kSegment = 256;
+
+__device__ __forceinline__ bool cut_here(u32 v) { return v * 0x9E3779B1u < 0xffffffffu / kSegment; }
+
+// succ[v] = node of v's first outgoing edge (0: none); the other edges' nodes get
+// their bit in `head`.  counts[0] += upper bound of the number of segments.
+__global__ void succ_kernel(const StreamView sv, u32 *__restrict__ succ, u32 *__restrict__ head,
+                            unsigned long long *__restrict__ counts) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= sv.n) return;
-    if (v == 0) {
-        P[0] = 0;
-        code[0] = 0;
-        len[0] = 0;
-        return;
+    u32 heads = 0;
+    if (v < sv.n) {
+        const u32 line = v / kLineBits, t = v - line * kLineBits + 32u;
+        u32 s = 0;
+        heads = v == 0 || cut_here(v);
+        for (u32 c = 0; c < 4u; c++) {
+            const ulonglong4 w = ld_line(sv.lines + (u64)c * sv.lpc + line);
+            if (!((sector_word(w, t >> 6) >> (63u - (t & 63u))) & 1ull)) continue;
+            const u32 x = sv.C[c] + line_rank_from(w, t - 32u);
+            if (s == 0) {
+                s = x;
+            } else {
+                atomicOr(head + (x >> 5), 1u << (x & 31u));
+                heads++;
+            }
+        }
+        succ[v] = s;
     }
-    u32 u = sv.pred(v);
-    if (u >= sv.n) {  // not an SBWT: record it, point at the root
-        atomicAdd(bad, 1ull);
-        u = 0;
-    }
-    P[v] = u;
-    code[v] = sv.last_letter(v);
-    len[v] = 1;
+    heads = __reduce_add_sync(0xffffffffu, heads);
+    if ((threadIdx.x & 31u) == 0 && heads) atomicAdd(counts, (unsigned long long)heads);
 }
 
-// One doubling round: window m -> 2m letters.
-__global__ void double_kernel(u32 n, u32 m, const u32 *__restrict__ P, const u64 *__restrict__ code,
-                              const uint8_t *__restrict__ len, u32 *__restrict__ P2, u64 *__restrict__ code2,
-                              uint8_t *__restrict__ len2) {
+// The segments' first nodes, in any order.
+__global__ void heads_kernel(u32 n, const u32 *__restrict__ head, u32 *__restrict__ first,
+                             unsigned long long *__restrict__ count) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const u32 l = len[v];
-    const u32 u = P[v];
-    if (l < m) {  // the chain reached the root inside the window
-        code2[v] = code[v];
-        len2[v] = (uint8_t)l;
-        P2[v] = 0;
-        return;
+    const bool is = v < n && (v == 0 || cut_here(v) || ((head[v >> 5] >> (v & 31u)) & 1u));
+    const u32 m = __ballot_sync(0xffffffffu, is);
+    if (!m) return;
+    unsigned long long base = 0;
+    if ((threadIdx.x & 31u) == 0) base = atomicAdd(count, (unsigned long long)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (is) first[base + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u))] = v;
+}
+
+__global__ void segment_len_kernel(u32 n_seg, const u32 *__restrict__ first, const u32 *__restrict__ succ,
+                                   u32 *__restrict__ len) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > n_seg) return;
+    u32 l = 0;
+    if (i < n_seg) {
+        u32 v = first[i];
+        do {
+            v = succ[v];
+            l++;
+        } while (v && !cut_here(v));
     }
-    code2[v] = code[v] | (code[u] << (2u * m));
-    len2[v] = (uint8_t)(m + len[u]);
-    P2[v] = P[u];
+    len[i] = l;  // len[n_seg] = 0: its prefix sum is the number of nodes reached
+}
+
+struct PathArrays {
+    u32 *node, *pos;    // path_node, node_pos
+    ulonglong2 *path;
+    u64 *code;          // letter t from the end of the label at bits 2t, 2t+1 (t < k)
+    uint8_t *len;       // letters of the label before its $ padding, at most k
+};
+
+// The segment of `count` nodes that starts at v goes to positions off .. off + count - 1.
+__device__ void write_segment(const StreamView &sv, u32 k, const u32 *succ, u32 v, u32 off, u32 count,
+                              const PathArrays &a, unsigned long long *bad) {
+    const u64 mask = k < 32u ? (1ull << (2u * k)) - 1ull : ~0ull;
+    u64 code = 0;
+    u32 l = 0;
+    for (u32 u = v; l < k && u; l++) {
+        code |= (u64)sv.last_letter(u) << (2u * l);
+        u = sv.pred(u);
+        if (u >= sv.n) {  // not an SBWT: record it, stop at the root
+            atomicAdd(bad, 1ull);
+            u = 0;
+        }
+    }
+    atomicOr((unsigned long long *)&a.path[off >> 5].y, 1ull << (63u - (off & 31u)));
+    for (u32 i = 0; i < count; i++) {
+        a.node[off + i] = v;
+        a.pos[v] = off + i;
+        a.code[v] = code;
+        a.len[v] = (uint8_t)l;
+        v = succ[v];
+        code = ((code << 2) | sv.last_letter(v)) & mask;
+        l = min(l + 1u, k);
+    }
+}
+
+__global__ void segment_write_kernel(const StreamView sv, u32 k, u32 n_seg, const u32 *__restrict__ first,
+                                     const u32 *__restrict__ succ, const u32 *__restrict__ off, const PathArrays a,
+                                     unsigned long long *__restrict__ bad) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_seg) write_segment(sv, k, succ, first[i], off[i], off[i + 1u] - off[i], a, bad);
+}
+
+// Cycles that no cut falls on (short ones): the thread of a cycle's smallest node writes it.
+__global__ void cycles_kernel(const StreamView sv, u32 k, const u32 *__restrict__ succ, const PathArrays a,
+                              u32 *__restrict__ reached, unsigned long long *__restrict__ bad) {
+    const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= sv.n || *(volatile u32 *)(a.pos + v) != ~0u) return;
+    u32 x = succ[v], count = 1;
+    for (; x > v; x = succ[x]) count++;
+    if (x == v) write_segment(sv, k, succ, v, atomicAdd(reached, count), count, a, bad);
+}
+
+// The last letters of the path's nodes, 32 positions a thread.
+__global__ void path_letters_kernel(const StreamView sv, const u32 *__restrict__ node, ulonglong2 *__restrict__ path,
+                                    u32 blocks) {
+    const u32 b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= blocks) return;
+    u64 x = 0, past = 0;
+    for (u32 t = 0; t < 32u; t++) {
+        const u64 i = (u64)b * 32u + t;
+        if (i < sv.n) x |= (u64)sv.last_letter(node[i]) << (62u - 2u * t);
+        else past |= 1ull << (63u - t);  // the last segment ends here
+    }
+    path[b].x = x;
+    path[b].y |= past;
 }
 
 // One thread per byte: the nibbles of nodes 2t and 2t+1.
@@ -98,19 +192,96 @@ __global__ void node_nibbles_kernel(u32 n, u32 k, const u64 *__restrict__ code, 
     node[t] = (uint8_t)byte;
 }
 
-// Backward table: entry v = pred(v) | group_letters(pred(v)) << 32 (node 0: 0).
-__global__ void back_table_kernel(const StreamView sv, u64 *__restrict__ back) {
+// ---- structures of the forward walk (WalkView, stream.cuh)
+
+// The q-mer bitmap: one atomic per distinct q-mer (labels are sorted, so equal
+// suffixes of q letters are neighbours).
+__global__ void qbits_kernel(u32 n, u32 q, const u64 *__restrict__ code, const uint8_t *__restrict__ len,
+                             u32 *__restrict__ qbits) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= sv.n) return;
-    u64 e = 0;
-    if (v) {
-        const u32 u0 = sv.pred(v);
-        if (u0 < sv.n) e = (u64)u0 | ((u64)sv.group_letters(u0) << 32);
+    if (v >= n || len[v] < q) return;
+    const u64 x = code[v] & ((1ull << (2u * q)) - 1ull);  // q <= 16
+    if (v && len[v - 1] >= q && (code[v - 1] & ((1ull << (2u * q)) - 1ull)) == x) return;
+    atomicOr(qbits + (x >> 5), 1u << (x & 31u));
+}
+
+__global__ void marks_kernel(u32 n, const uint8_t *__restrict__ node, u32 *__restrict__ marks, u32 words) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= words) return;
+    u32 w = 0;
+    for (u32 b = 0; b < 32u; b++) {
+        const int64_t v = (int64_t)i * kMarkCols - 4 + b;
+        if (v < 0 || v >= (int64_t)n) continue;
+        if ((node[v >> 1] >> ((v & 1) * 4)) & kGroupStart) w |= 1u << b;
     }
-    back[v] = e;
+    marks[i] = w;
+}
+
+// code[v] -> the node's key, in place; ~0 past the last node.
+__global__ void keys_kernel(u32 n, u32 n_pad, u32 k, u64 *__restrict__ code, const uint8_t *__restrict__ len) {
+    const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n_pad) return;
+    u64 x = ~0ull;
+    if (v < n) {
+        x = letters_reverse(code[v]);
+        if (k < 32u) {
+            x &= ~0ull << (64u - 2u * k);
+            if (len[v] >= k) x |= 1ull;
+        }
+    }
+    code[v] = x;
+}
+
+// What the forward walk relies on, for every column: keys ascend, strictly
+// between labels without $; only group starts have outgoing edges; a group has
+// at most 5 members.  An index whose k is not the one it was built for fails.
+__global__ void walk_check_kernel(u32 n, u32 k, const u64 *__restrict__ keys, const uint8_t *__restrict__ node,
+                                  const u32 *__restrict__ marks, const ulonglong4 *__restrict__ lines, u32 lpc,
+                                  unsigned long long *__restrict__ bad) {
+    const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const u32 f = (u32)(node[v >> 1] >> ((v & 1u) * 4u)) & 15u;
+    bool ok = true;
+    if (v + 1u < n) {
+        const u64 a = keys[v], b = keys[v + 1u];
+        const u32 g = (u32)(node[(v + 1u) >> 1] >> (((v + 1u) & 1u) * 4u)) & 15u;
+        ok = a < b || (a == b && !((f & 7u) && (g & 7u)));
+    }
+    if (!(f & kGroupStart)) {
+        ok = ok && v - group_start(marks[v / kMarkCols], v) < 5u;
+        const u32 line = v / kLineBits, t = v - line * kLineBits + 32u;
+        for (u32 c = 0; c < 4u; c++)
+            ok = ok && !((sector_word(lines[(u64)c * lpc + line], t >> 6) >> (63u - (t & 63u))) & 1ull);
+    }
+    if (!ok) atomicAdd(bad, 1ull);
+}
+
+// Letters of the q-mers: the smallest q with 4^q >= 4 n, so that at most a
+// quarter of the q-mers of random letters are present, as long as the bitmap
+// (4^q bits) is no larger than 32 MiB (q = 14), where it stays in L2 next to
+// the lines; larger indexes keep q = 14 up to 4^14 columns, then take the
+// smallest q with 4^q > n.
+u32 walk_q(u64 n, u32 k) {
+    u32 q = 1;
+    while (q < 14u && (1ull << (2u * q)) < 4ull * n) q++;
+    while (q < 16u && (1ull << (2u * q)) < n) q++;
+    return q < k ? q : k;
 }
 
 }  // namespace
+
+WalkView walk_view(const sbwt_index *ix) {
+    WalkView w;
+    w.labels = ix->d_labels;
+    w.qbits = ix->d_qbits;
+    w.marks = ix->d_marks;
+    w.path_node = ix->d_path_node;
+    w.node_pos = ix->d_node_pos;
+    w.path = ix->d_path;
+    w.q = ix->walk_q;
+    w.n = (u32)ix->n;
+    return w;
+}
 
 StreamView stream_view(const sbwt_index *ix) {
     StreamView sv;
@@ -124,16 +295,31 @@ StreamView stream_view(const sbwt_index *ix) {
         sv.C[c] = (u32)ix->C[c];
     }
     sv.node = ix->d_node;
-    sv.back = ix->d_back;
     sv.n = (u32)ix->n;
     return sv;
+}
+
+void free_walk(sbwt_index *ix) {
+    cudaFree(ix->d_labels);
+    cudaFree(ix->d_qbits);
+    cudaFree(ix->d_marks);
+    cudaFree(ix->d_path_node);
+    cudaFree(ix->d_node_pos);
+    cudaFree(ix->d_path);
+    ix->d_labels = nullptr;
+    ix->d_qbits = nullptr;
+    ix->d_marks = nullptr;
+    ix->d_path_node = nullptr;
+    ix->d_node_pos = nullptr;
+    ix->d_path = nullptr;
+    ix->walk_q = 0;
 }
 
 int build_stream(sbwt_index *ix, cudaStream_t s) {
     if (ix->stream_ok) return 0;
     if (!ix->lines_ok) return set_error("the backward step needs the line layout");
     if (ix->k > 32 || ix->k < 2) return set_error("k out of range");
-    const u32 n = (u32)ix->n;
+    const u32 n = (u32)ix->n, k = ix->k;
     u64 total = 0;
     for (int c = 0; c < 4; c++) {
         const u64 ones = ix->C[c + 1] - ix->C[c];
@@ -141,70 +327,91 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
         ix->sel_n[c] = (u32)((ones + 63) >> kSelLog);
         total += ix->sel_n[c] + 1;
     }
-    SBWT_CHECK_CUDA(cudaMalloc(&ix->d_sel, total * sizeof(u32)));
-    SBWT_CHECK_CUDA(cudaMemsetAsync(ix->d_sel, 0, total * sizeof(u32), s));
-    SBWT_CHECK_CUDA(cudaMalloc(&ix->d_node, (size_t)n / 2 + 16));
-    for (int c = 0; c < 4; c++) {
-        if (!ix->sel_n[c]) continue;
-        select_samples_kernel<<<(ix->lpc + 255) / 256, 256, 0, s>>>(ix->d_lines + (u64)c * ix->lpc, ix->lpc,
-                                                                     ix->d_sel + ix->sel_off[c], ix->sel_n[c]);
-        SBWT_CHECK_CUDA(cudaGetLastError());
-    }
-    // scratch: P, code, len twice, plus a flag
-    u32 *P[2] = {nullptr, nullptr};
-    u64 *code[2] = {nullptr, nullptr};
-    uint8_t *len[2] = {nullptr, nullptr};
-    unsigned long long *bad = nullptr;
-    int rc = 0;
-    auto fail = [&](cudaError_t e) {
-        rc = set_error("CUDA error while building the backward-step structures: %s", cudaGetErrorString(e));
-    };
+    const u32 n_pad = (n + 3u) / 4u * 4u + 4u;
+    const u32 q = walk_q(n, k), mark_words = n / kMarkCols + 1u, path_blocks = n / 32u + 2u;
+    const size_t qwords = std::max<size_t>(1, (size_t)((1ull << (2u * q)) / 32u));
+    const u32 blocks = (n + 255) / 256;
+    // scratch: first successors, head bits, label lengths, segments; counters: segments (upper bound),
+    // segments, nodes without a predecessor, columns the forward walk cannot take
+    u32 *succ = nullptr, *head = nullptr, *first = nullptr, *off = nullptr;
+    uint8_t *len = nullptr;
+    void *tmp = nullptr;
+    unsigned long long *cnt = nullptr, h_cnt[4] = {0, 0, 0, 0};
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 2 && e == cudaSuccess; i++) {
-        e = cudaMalloc(&P[i], (size_t)n * sizeof(u32));
-        if (e == cudaSuccess) e = cudaMalloc(&code[i], (size_t)n * sizeof(u64));
-        if (e == cudaSuccess) e = cudaMalloc(&len[i], (size_t)n);
-    }
-    if (e == cudaSuccess) e = cudaMalloc(&bad, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) {
-        fail(e);
-    } else {
-        ix->stream_ok = false;
+    auto ok = [&](cudaError_t x) {
+        if (e == cudaSuccess) e = x;
+        return e == cudaSuccess;
+    };
+    int rc = 0;
+    do {
+        if (!ok(cudaMalloc(&ix->d_sel, total * sizeof(u32))) || !ok(cudaMalloc(&ix->d_node, (size_t)n / 2 + 16)) ||
+            !ok(cudaMalloc(&ix->d_labels, (size_t)n_pad * sizeof(u64))) ||
+            !ok(cudaMalloc(&ix->d_qbits, qwords * sizeof(u32))) ||
+            !ok(cudaMalloc(&ix->d_marks, (size_t)mark_words * sizeof(u32))) ||
+            !ok(cudaMalloc(&ix->d_path_node, (size_t)n * sizeof(u32))) ||
+            !ok(cudaMalloc(&ix->d_node_pos, (size_t)n * sizeof(u32))) ||
+            !ok(cudaMalloc(&ix->d_path, (size_t)path_blocks * sizeof(ulonglong2))) ||
+            !ok(cudaMalloc(&succ, (size_t)n * sizeof(u32))) || !ok(cudaMalloc(&head, ((size_t)n / 32 + 1) * sizeof(u32))) ||
+            !ok(cudaMalloc(&len, n)) || !ok(cudaMalloc(&cnt, sizeof h_cnt)))
+            break;
+        cudaMemsetAsync(ix->d_sel, 0, total * sizeof(u32), s);
+        cudaMemsetAsync(ix->d_qbits, 0, qwords * sizeof(u32), s);
+        cudaMemsetAsync(ix->d_node_pos, 0xff, (size_t)n * sizeof(u32), s);
+        cudaMemsetAsync(ix->d_path, 0, (size_t)path_blocks * sizeof(ulonglong2), s);
+        cudaMemsetAsync(head, 0, ((size_t)n / 32 + 1) * sizeof(u32), s);
+        cudaMemsetAsync(cnt, 0, sizeof h_cnt, s);
+        for (int c = 0; c < 4; c++)
+            if (ix->sel_n[c])
+                select_samples_kernel<<<(ix->lpc + 255) / 256, 256, 0, s>>>(
+                    ix->d_lines + (u64)c * ix->lpc, ix->lpc, ix->d_sel + ix->sel_off[c], ix->sel_n[c]);
         const StreamView sv = stream_view(ix);
-        const u32 blocks = (n + 255) / 256;
-        pred_init_kernel<<<blocks, 256, 0, s>>>(sv, P[0], code[0], len[0], bad);
-        int cur = 0;
-        for (u32 m = 1; m <= 16; m <<= 1) {
-            double_kernel<<<blocks, 256, 0, s>>>(n, m, P[cur], code[cur], len[cur], P[cur ^ 1], code[cur ^ 1],
-                                                 len[cur ^ 1]);
-            cur ^= 1;
-        }
-        node_nibbles_kernel<<<(n / 2 + 1 + 255) / 256, 256, 0, s>>>(n, ix->k, code[cur], len[cur], ix->d_node);
-        if (SBWT_BACK_TABLE) {
-            e = cudaMalloc(&ix->d_back, (size_t)n * sizeof(u64));
-            if (e == cudaSuccess) back_table_kernel<<<blocks, 256, 0, s>>>(stream_view(ix), ix->d_back);
-        }
-        unsigned long long h_bad = 0;
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h_bad, bad, sizeof h_bad, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) fail(e);
-        else if (h_bad) rc = set_error("the bit vectors are not an SBWT: %llu nodes have no predecessor", h_bad);
-    }
-    for (int i = 0; i < 2; i++) {
-        cudaFree(P[i]);
-        cudaFree(code[i]);
-        cudaFree(len[i]);
-    }
-    cudaFree(bad);
+        succ_kernel<<<blocks, 256, 0, s>>>(sv, succ, head, cnt);
+        if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
+            break;
+        const u32 max_seg = (u32)h_cnt[0];
+        if (!ok(cudaMalloc(&first, (size_t)max_seg * sizeof(u32))) || !ok(cudaMalloc(&off, ((size_t)max_seg + 1) * sizeof(u32))))
+            break;
+        heads_kernel<<<blocks, 256, 0, s>>>(n, head, first, cnt + 1);
+        if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
+            break;
+        const u32 n_seg = (u32)h_cnt[1];
+        segment_len_kernel<<<n_seg / 128 + 1, 128, 0, s>>>(n_seg, first, succ, off);
+        size_t tmp_bytes = 0;
+        if (!ok(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, off, off, (int64_t)n_seg + 1, s)) ||
+            !ok(cudaMalloc(&tmp, tmp_bytes ? tmp_bytes : 1)) ||
+            !ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, off, off, (int64_t)n_seg + 1, s)))
+            break;
+        const PathArrays pa{ix->d_path_node, ix->d_node_pos, ix->d_path, ix->d_labels, len};
+        segment_write_kernel<<<n_seg / 128 + 1, 128, 0, s>>>(sv, k, n_seg, first, succ, off, pa, cnt + 2);
+        cycles_kernel<<<blocks, 256, 0, s>>>(sv, k, succ, pa, off + n_seg, cnt + 2);
+        path_letters_kernel<<<(path_blocks + 255) / 256, 256, 0, s>>>(sv, ix->d_path_node, ix->d_path, path_blocks);
+        node_nibbles_kernel<<<(n / 2 + 1 + 255) / 256, 256, 0, s>>>(n, k, ix->d_labels, len, ix->d_node);
+        qbits_kernel<<<blocks, 256, 0, s>>>(n, q, ix->d_labels, len, ix->d_qbits);
+        marks_kernel<<<(mark_words + 255) / 256, 256, 0, s>>>(n, ix->d_node, ix->d_marks, mark_words);
+        keys_kernel<<<(n_pad + 255) / 256, 256, 0, s>>>(n, n_pad, k, ix->d_labels, len);
+        walk_check_kernel<<<blocks, 256, 0, s>>>(n, k, ix->d_labels, ix->d_node, ix->d_marks, ix->d_lines, ix->lpc,
+                                                 cnt + 3);
+        if (!ok(cudaGetLastError()) || !ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) ||
+            !ok(cudaStreamSynchronize(s)))
+            break;
+        if (h_cnt[2]) rc = set_error("the bit vectors are not an SBWT: %llu nodes have no predecessor", h_cnt[2]);
+    } while (false);
+    if (e != cudaSuccess)
+        rc = set_error("CUDA error while building the walk's structures: %s", cudaGetErrorString(e));
+    cudaFree(succ);
+    cudaFree(head);
+    cudaFree(first);
+    cudaFree(off);
+    cudaFree(len);
+    cudaFree(tmp);
+    cudaFree(cnt);
+    if (rc || h_cnt[3]) free_walk(ix);  // with h_cnt[3], reads are searched without the forward walk
+    else ix->walk_q = q;
     if (rc) {
         cudaFree(ix->d_node);
         cudaFree(ix->d_sel);
-        cudaFree(ix->d_back);
         ix->d_node = nullptr;
         ix->d_sel = nullptr;
-        ix->d_back = nullptr;
         return rc;
     }
     ix->stream_ok = true;

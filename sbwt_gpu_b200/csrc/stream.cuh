@@ -27,12 +27,6 @@ constexpr u32 kSelLog = 6;          // one select sample per 64 ones
 constexpr uint8_t kGroupStart = 8;  // node nibble: bit 3 = first node of its group
 constexpr u32 kNoNode = 0;          // node 0 (the all-$ root) is never a k-mer's node
 
-// Backward steps through the 8-byte-per-column backward table (1) or through
-// select + node nibbles (0).
-#ifndef SBWT_BACK_TABLE
-#define SBWT_BACK_TABLE 1
-#endif
-
 // Position of the (i+1)-th one (0-based i) of the 64-bit MSB-first word w.
 __device__ __forceinline__ u32 msb_select(u64 w, u32 i) {
     u32 pos = 0;
@@ -90,7 +84,6 @@ struct StreamView {
     u32 sel_off[4];
     u32 sel_n[4];
     const uint8_t *node;   // per node a nibble (first letter | kGroupStart), two per byte
-    const u64 *back;       // backward table: per node pred(v) | group_letters(pred(v)) << 32
     u32 n;                 // nodes
     u32 C[4];
 
@@ -105,32 +98,8 @@ struct StreamView {
         return line_select(lines + (u64)b * lpc, lpc, sel + sel_off[b], sel_n[b], v - cb);
     }
 
-    // Letters present as first letters in the group that starts at u0 (bit 0 = $, bit 1 + c = letter c).
-    __device__ __forceinline__ u32 group_letters(u32 u0) const {
-        u32 m = 0;
-        u32 u = u0;
-#pragma unroll 1
-        for (u32 g = 0; g < 5u && u < n; g++, u++) {
-            const u32 f = (u32)(__ldg(node + (u >> 1)) >> ((u & 1u) << 2)) & 15u;
-            if (g && (f & kGroupStart)) break;
-            m |= 1u << (f & 7u);
-        }
-        return m;
-    }
-
-#if SBWT_BACK_TABLE
-    // Node of the k-mer a.y given the node v of the k-mer y.b, or kNoNode: one
-    // load of v's entry u0 | group_letters(u0) << 32 (the backward table); the
-    // member with first letter a sits after the members with smaller ones.
-    __device__ __forceinline__ u32 back_step(u32 v, u32 a, bool ef, u64 pol) const {
-        const u64 e = ld_gather_u64(back + v, ef, pol);
-        const u32 m = (u32)(e >> 32);
-        if (!((m >> (a + 1u)) & 1u)) return kNoNode;
-        return (u32)e + (u32)__popc(m & ((1u << (a + 1u)) - 1u));
-    }
-#else
     // Node of the k-mer a.y given the node v of the k-mer y.b, or kNoNode.
-    __device__ __forceinline__ u32 back_step(u32 v, u32 a, bool, u64) const {
+    __device__ __forceinline__ u32 back_step(u32 v, u32 a) const {
         u32 u = pred(v);
         if (u >= n) return kNoNode;
         const u32 want = a + 1u;
@@ -144,8 +113,50 @@ struct StreamView {
         }
         return kNoNode;
     }
-#endif
 };
+
+// ------------------------------------------------------- the forward walk
+//
+// Structures of the forward walk (walk.cu), built by stream.cu:
+//  * labels: per node its last k letters as a colex key (last letter in the
+//    top two bits), so that the array is sorted; bit 0 is set on labels without
+//    $ when k < 32 (a $ counts as A otherwise).  Padded to whole groups of 4
+//    with ~0.
+//  * qbits: bit i = the q-mer of code i (first letter in the top two of 2q bits)
+//    is the suffix of some label, i.e. a substring of an indexed k-mer.
+//  * marks: group starts.  Word i holds columns 28 i - 4 .. 28 i + 27 (bit b =
+//    column 28 i - 4 + b), so one word gives the group start of any column: a
+//    group has at most 5 members.
+//  * paths: every node once, in segments along edges: path_node[i + 1] is the
+//    first successor of path_node[i] unless position i + 1 starts a segment.
+//    node_pos is the inverse.  path[b] holds positions 32 b .. 32 b + 31: x =
+//    the last letters of their labels (MSB-first), y = segment starts (position
+//    32 b + t at bit 63 - t).  A read that follows the graph is compared with a
+//    path 32 letters at a time, and its answers lie in order in path_node.
+struct WalkView {
+    const u64 *labels;
+    const u32 *qbits;
+    const u32 *marks;
+    const u32 *path_node;
+    const u32 *node_pos;
+    const ulonglong2 *path;
+    u32 q;  // letters of the q-mers, 0: the structures are not there
+    u32 n;
+};
+
+constexpr u32 kMarkCols = 28;
+
+// Reverses the order of the 32 2-bit letters of a word.
+__device__ __forceinline__ u64 letters_reverse(u64 x) {
+    x = __brevll(x);
+    return ((x >> 1) & 0x5555555555555555ull) | ((x & 0x5555555555555555ull) << 1);
+}
+
+// First column of the group of column v.
+__device__ __forceinline__ u32 group_start(u32 w, u32 v) {
+    const u32 b = v % kMarkCols + 4u;  // w = marks[v / 28]
+    return v - (u32)__clz((int)(w << (31u - b)));
+}
 
 }  // namespace dev
 }  // namespace sbwt

@@ -1,0 +1,96 @@
+"""The forward walk (walk.cu) where it can go wrong, against the oracle: paths that are cycles, keys
+that tie with the labels of dummy nodes, batches on both sides of its batch-size rules, unaligned
+answers, and an index searched with another k than its own."""
+import numpy as np
+import pytest
+
+import oracle as orc
+import sbwt_gpu_b200 as sg
+from sbwt_gpu_b200 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def _seqs(kind, k, rng):
+    g = wl.random_bases(rng, 3000).tobytes().decode()
+    if kind == "cycles":  # closed paths: one letter, two letters, a longer period, a circle of the genome
+        return ["A" * 80, "CT" * 60, "ACGGT" * 40, g[:700] + g[:700]]
+    if kind == "ties":  # keys of A-runs tie with $-padded labels, keys of T-runs with the padding
+        return ["A" * (k + 5) + g[:200], "T" * (k + 7), "CA" + "A" * k, g[200:260] + "T" * (k + 1), "AC" * k]
+    return [g, g[:1500] + "G" + g[1501:], g[900:1000]]  # "branches"
+
+
+def _rows(parts):
+    starts = np.zeros(len(parts) + 1, dtype=np.uint64)
+    starts[1:] = np.cumsum([len(p) for p in parts])
+    return np.frombuffer("".join(parts).encode(), dtype=np.uint8), starts
+
+
+def _search(ix, letters, rows, nk, shift=0):
+    import torch
+    d_l = torch.from_numpy(letters.copy()).cuda()
+    d_r = torch.from_numpy(rows.view(np.int64)).cuda()
+    ans = torch.full((nk + 8,), -7, dtype=torch.int64, device="cuda")
+    bits = torch.zeros((nk + 31) // 32 + 1, dtype=torch.int32, device="cuda")
+    ix.search_reads(d_l, d_r, ans[shift:shift + nk], nk, d_member_bits=bits)
+    mem = torch.zeros_like(bits)
+    ix.search_reads(d_l, d_r, None, nk, d_member_bits=mem)
+    torch.cuda.synchronize()
+    a = ans.cpu().numpy()
+    assert (a[:shift] == -7).all() and (a[shift + nk:] == -7).all()
+    assert torch.equal(bits, mem)
+    a = a[shift:shift + nk].view(np.uint64)
+    want = np.zeros((nk + 31) // 32 * 32, dtype=np.uint8)
+    want[:nk] = a != orc.NOT_FOUND
+    got = bits.cpu().numpy().view(np.uint32)[: (nk + 31) // 32]
+    assert np.array_equal(got, np.packbits(want, bitorder="little").view(np.uint32))
+    return a
+
+
+@pytest.mark.parametrize("k,p", [(4, 2), (11, 0), (16, 8), (31, 10), (32, 12)])
+@pytest.mark.parametrize("kind", ["cycles", "ties", "branches"])
+def test_walk_equals_the_oracle(cuda, kind, k, p):
+    rng = wl.rng_for(1000 + k)
+    seqs = _seqs(kind, k, rng)
+    built = sg.build_sbwt([s.encode() for s in seqs], k)
+    text = "".join(seqs)
+    parts = list(seqs)
+    for n in [1, k - 1, k, k + 1, 64, 255, 256, 257, 511, 600]:
+        at = int(rng.integers(0, max(1, len(text) - n)))
+        read = bytearray(text[at:at + n].encode())
+        for i in rng.integers(0, len(read), size=len(read) // 60):
+            read[i] = int(wl.ACGT[rng.integers(0, 4)])
+        parts += [text[at:at + n], read.decode(), wl.random_bases(rng, n).tobytes().decode(), ""]
+    letters, rows = _rows(parts)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, p)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        for shift in (0, 1, 3):
+            assert np.array_equal(_search(ix, letters, rows, want.size, shift), want)
+
+
+@pytest.mark.parametrize("reads", [70_000, 70_500])  # below and above the batch that is filled ahead
+def test_walk_batch_sizes(cuda, reads):
+    rng = wl.rng_for(77)
+    k, p = 31, 10
+    genome = wl.random_bases(rng, 50_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, reads // 4, reads - reads // 4, 149, 0.01)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, p)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        assert np.array_equal(_search(ix, letters, rows, want.size, 1), want)
+
+
+@pytest.mark.parametrize("dk", [-2, 1])
+def test_another_k_than_the_index(cuda, dk):
+    """Searched with a k that is not the one of its labels, an index takes the walk without the labels; the
+    answers are those of one search per k-mer."""
+    rng = wl.rng_for(5)
+    k = 21 + dk
+    genome = wl.random_bases(rng, 20_000)
+    built = sg.build_sbwt([genome.tobytes(), genome[:500].tobytes()], 21)
+    letters, rows = wl.mixed_reads(rng, genome, 60, 60, 150, 0.01)
+    nk = sg.count_kmers(rows, k)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=8) as ix:
+        got = _search(ix, letters, rows, nk)
+        ix.set_search_mode(sg.SEARCH_EVERY_KMER)
+        assert np.array_equal(got, _search(ix, letters, rows, nk))
