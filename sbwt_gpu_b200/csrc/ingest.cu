@@ -15,44 +15,86 @@ using namespace dev;
 // only 'C'/'c' become 0x63, 'G'/'g' 0x67, 'T'/'t' 0x74.  The multiply by
 // 0x40100401 moves the code of byte i to bits 30-2i..31-2i without carries
 // into the top byte.
-__device__ __forceinline__ u32 pack4(u32 x) {
+__device__ __forceinline__ u32 pack4_any(u32 x) {
     const u32 lo = x | 0x20202020u;
     const u32 codes = (__vcmpeq4(lo, 0x63636363u) & 0x01010101u) | (__vcmpeq4(lo, 0x67676767u) & 0x02020202u) |
                       (__vcmpeq4(lo, 0x74747474u) & 0x03030303u);
     return (codes * 0x40100401u) >> 24;
 }
 
-__device__ __forceinline__ u64 pack8x4(const uint4 &v0, const uint4 &v1) {
-    return ((u64)pack4(v0.x) << 56) | ((u64)pack4(v0.y) << 48) | ((u64)pack4(v0.z) << 40) |
-           ((u64)pack4(v0.w) << 32) | ((u64)pack4(v1.x) << 24) | ((u64)pack4(v1.y) << 16) |
-           ((u64)pack4(v1.z) << 8) | (u64)pack4(v1.w);
+// The same where all four are ACGT or acgt: their low three bits (1, 3, 7, 4)
+// select the code and the letter they then have to be from two 8-byte tables
+// held in registers.  bad != 0 afterwards: some byte is none of them.
+__device__ __forceinline__ u32 pack4(u32 x, u32 &bad) {
+    const u32 t = x & 0x07070707u;
+    const u32 sel = __byte_perm(t | (t >> 4), 0, 0x4420);  // the four indices as nibbles
+    bad |= __byte_perm(0x630061ffu, 0x67ffff74u, sel) ^ (x | 0x20202020u);
+    return (__byte_perm(0x01000000u, 0x02000003u, sel) * 0x40100401u) >> 24;
 }
 
-// One thread per output word (32 letters), two 16-byte loads when the word
-// lies wholly inside the letters; the word holding the end, and the padding
-// words after it, are assembled byte by byte (bytes past n_letters are 0,
-// i.e. 'A', as the reference's zero padding, kmer_search.hpp:292-301).
-__global__ void pack_kernel(const uint8_t *__restrict__ letters, u64 n_letters, u64 *__restrict__ words, u64 n_words,
-                            bool aligned) {
-    const u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n_words) return;
-    const u64 first = w * 32u;
-    if (aligned && first + 32u <= n_letters) {
-        const uint4 *p = reinterpret_cast<const uint4 *>(letters + first);
-        words[w] = pack8x4(__ldg(p), __ldg(p + 1));
-        return;
-    }
+__device__ __forceinline__ u64 pack32(const uint4 &v0, const uint4 &v1) {
+    const u32 in[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    u32 bad = 0;
     u64 x = 0;
-    for (u32 g = 0; g < 8; g++) {
-        u32 v = 0;
-        for (u32 b = 0; b < 4; b++) {
-            const u64 i = first + g * 4u + b;
-            const u32 ch = i < n_letters ? (u32)letters[i] : 0u;
-            v |= ch << (8 * b);
-        }
-        x |= (u64)pack4(v) << (56 - 8 * g);
+#pragma unroll
+    for (u32 i = 0; i < 8u; i++) x |= (u64)pack4(in[i], bad) << (56u - 8u * i);
+    if (bad) {
+        x = 0;
+#pragma unroll
+        for (u32 i = 0; i < 8u; i++) x |= (u64)pack4_any(in[i]) << (56u - 8u * i);
     }
-    words[w] = x;
+    return x;
+}
+
+// kPackWords output words (32 letters each) per thread, a block apart.  ALIGN:
+// the letters' alignment, 32 (one load a word), 16 (two) or 1; the words that
+// hold the end, the padding after it and all unaligned ones are assembled byte
+// by byte (bytes past n_letters are 0, i.e. 'A', as the reference's zero
+// padding, kmer_search.hpp:292-301).  HBM-bound: 1.25 bytes a letter.  1.5G
+// letters: 0.28 ms (6.8 TB/s) with 32-byte loads and the table form of pack4,
+// 0.31 with two 16-byte loads and one word a thread; byte compares for every
+// letter took 0.47.
+constexpr u32 kPackThreads = 256, kPackWords = 4;
+
+template <int ALIGN>
+__global__ void __launch_bounds__(kPackThreads) pack_kernel(const uint8_t *__restrict__ letters, u64 n_letters,
+                                                            u64 *__restrict__ words, u64 n_words) {
+    const u64 w0 = (u64)blockIdx.x * (kPackThreads * kPackWords) + threadIdx.x;
+    const u64 whole = ALIGN == 1 ? 0 : n_letters / 32u;
+    uint4 v[kPackWords][2];
+#pragma unroll
+    for (u32 i = 0; i < kPackWords; i++) {
+        const u64 w = w0 + i * kPackThreads;
+        if (w >= whole) continue;
+        const uint4 *p = reinterpret_cast<const uint4 *>(letters + w * 32u);
+        if constexpr (ALIGN == 32) {
+            asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=r"(v[i][0].x), "=r"(v[i][0].y), "=r"(v[i][0].z), "=r"(v[i][0].w), "=r"(v[i][1].x), "=r"(v[i][1].y),
+                  "=r"(v[i][1].z), "=r"(v[i][1].w)
+                : "l"(p));
+        } else {
+            v[i][0] = __ldg(p);
+            v[i][1] = __ldg(p + 1);
+        }
+    }
+#pragma unroll
+    for (u32 i = 0; i < kPackWords; i++) {
+        const u64 w = w0 + i * kPackThreads;
+        if (w < whole) {
+            words[w] = pack32(v[i][0], v[i][1]);
+        } else if (w < n_words) {
+            u64 x = 0;
+            for (u32 g = 0; g < 8; g++) {
+                u32 c = 0;
+                for (u32 b = 0; b < 4; b++) {
+                    const u64 j = w * 32u + g * 4u + b;
+                    c |= (j < n_letters ? (u32)letters[j] : 0u) << (8 * b);
+                }
+                x |= (u64)pack4_any(c) << (56 - 8 * g);
+            }
+            words[w] = x;
+        }
+    }
 }
 
 struct KstartScan {
@@ -111,9 +153,10 @@ __global__ void member_bits_kernel(const u64 *__restrict__ answers, u64 n, uint3
 
 int launch_pack(const uint8_t *d_letters, uint64_t n_letters, uint64_t *d_words, cudaStream_t s) {
     const u64 n_words = (n_letters + 32u + 31u) / 32u;  // ceil((n+32)/32), kmer_search.hpp:294
-    const bool aligned = ((uintptr_t)d_letters & 15u) == 0;
-    const unsigned blocks = (unsigned)((n_words + 255) / 256);
-    pack_kernel<<<blocks, 256, 0, s>>>(d_letters, n_letters, d_words, n_words, aligned);
+    const uintptr_t at = (uintptr_t)d_letters;
+    const auto kern = at % 32u == 0 ? pack_kernel<32> : at % 16u == 0 ? pack_kernel<16> : pack_kernel<1>;
+    const u64 per = kPackThreads * kPackWords;
+    kern<<<(unsigned)((n_words + per - 1) / per), kPackThreads, 0, s>>>(d_letters, n_letters, d_words, n_words);
     SBWT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -38,9 +38,9 @@ __global__ void select_samples_kernel(const ulonglong4 *__restrict__ lines, u32 
     for (u32 s = s_lo; s <= s_hi && s < n_samples; s++) sel[s] = t;
 }
 
-// ---- paths: each column's first outgoing edge links it to one successor, and
-// every node but the root has one incoming edge, so the links form chains and
-// cycles.  They are cut into segments at the nodes without a link to them and at
+// ---- paths: each column's first outgoing edge links it to one successor (the
+// root's none: it has no letter), and every node but the root has one incoming
+// edge, so the links form chains and cycles.  They are cut into segments at the nodes without a link to them and at
 // one node in kSegment (by a hash), so that one thread per segment walks it: once
 // to size it, once to write it together with the labels, which roll along the
 // segment from its first node's (k select steps back).
@@ -50,8 +50,9 @@ constexpr u32 kSegment = 256;
 __device__ __forceinline__ bool cut_here(u32 v) { return v * 0x9E3779B1u < 0xffffffffu / kSegment; }
 
 // succ[v] = node of v's first outgoing edge (0: none); the other edges' nodes get
-// their bit in `head`.  counts[0] += upper bound of the number of segments.
-__global__ void succ_kernel(const StreamView sv, u32 *__restrict__ succ, u32 *__restrict__ head,
+// their bit in `head`, and v its bit in `fork` if there are any.  counts[0] +=
+// upper bound of the number of segments.
+__global__ void succ_kernel(const StreamView sv, u32 *__restrict__ succ, u32 *__restrict__ head, u32 *__restrict__ fork,
                             unsigned long long *__restrict__ counts) {
     const u32 v = blockIdx.x * blockDim.x + threadIdx.x;
     u32 heads = 0;
@@ -63,10 +64,11 @@ __global__ void succ_kernel(const StreamView sv, u32 *__restrict__ succ, u32 *__
             const ulonglong4 w = ld_line(sv.lines + (u64)c * sv.lpc + line);
             if (!((sector_word(w, t >> 6) >> (63u - (t & 63u))) & 1ull)) continue;
             const u32 x = sv.C[c] + line_rank_from(w, t - 32u);
-            if (s == 0) {
+            if (s == 0 && v) {
                 s = x;
             } else {
                 atomicOr(head + (x >> 5), 1u << (x & 31u));
+                atomicOr(fork + (v >> 5), 1u << (v & 31u));
                 heads++;
             }
         }
@@ -154,19 +156,26 @@ __global__ void cycles_kernel(const StreamView sv, u32 k, const u32 *__restrict_
     if (x == v) write_segment(sv, k, succ, v, atomicAdd(reached, count), count, a, bad);
 }
 
-// The last letters of the path's nodes, 32 positions a thread.
-__global__ void path_letters_kernel(const StreamView sv, const u32 *__restrict__ node, ulonglong2 *__restrict__ path,
-                                    u32 blocks) {
+// The last letters of the path's nodes, 32 positions a thread, and the positions that cannot be judged by the
+// letters alone: segment starts, and the positions after a node with more than one edge.
+__global__ void path_letters_kernel(const StreamView sv, const u32 *__restrict__ node, const u32 *__restrict__ fork,
+                                    ulonglong2 *__restrict__ path, u32 blocks) {
     const u32 b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= blocks) return;
-    u64 x = 0, past = 0;
+    u64 x = 0, starts = path[b].y, open = 0;
+    u32 u = b && (u64)b * 32u <= sv.n ? node[(u64)b * 32u - 1u] : 0u;  // the node before position 32 b
     for (u32 t = 0; t < 32u; t++) {
         const u64 i = (u64)b * 32u + t;
-        if (i < sv.n) x |= (u64)sv.last_letter(node[i]) << (62u - 2u * t);
-        else past |= 1ull << (63u - t);  // the last segment ends here
+        if ((fork[u >> 5] >> (u & 31u)) & 1u) open |= 1ull << (31u - t);
+        if (i < sv.n) {
+            u = node[i];
+            x |= (u64)sv.last_letter(u) << (62u - 2u * t);
+        } else {
+            starts |= 1ull << (63u - t);  // the last segment ends here
+        }
     }
     path[b].x = x;
-    path[b].y |= past;
+    path[b].y = starts | starts >> 32 | open;
 }
 
 // One thread per byte: the nibbles of nodes 2t and 2t+1.
@@ -333,7 +342,7 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
     const u32 blocks = (n + 255) / 256;
     // scratch: first successors, head bits, label lengths, segments; counters: segments (upper bound),
     // segments, nodes without a predecessor, columns the forward walk cannot take
-    u32 *succ = nullptr, *head = nullptr, *first = nullptr, *off = nullptr;
+    u32 *succ = nullptr, *head = nullptr, *fork = nullptr, *first = nullptr, *off = nullptr;
     uint8_t *len = nullptr;
     void *tmp = nullptr;
     unsigned long long *cnt = nullptr, h_cnt[4] = {0, 0, 0, 0};
@@ -352,6 +361,7 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
             !ok(cudaMalloc(&ix->d_node_pos, (size_t)n * sizeof(u32))) ||
             !ok(cudaMalloc(&ix->d_path, (size_t)path_blocks * sizeof(ulonglong2))) ||
             !ok(cudaMalloc(&succ, (size_t)n * sizeof(u32))) || !ok(cudaMalloc(&head, ((size_t)n / 32 + 1) * sizeof(u32))) ||
+            !ok(cudaMalloc(&fork, ((size_t)n / 32 + 1) * sizeof(u32))) ||
             !ok(cudaMalloc(&len, n)) || !ok(cudaMalloc(&cnt, sizeof h_cnt)))
             break;
         cudaMemsetAsync(ix->d_sel, 0, total * sizeof(u32), s);
@@ -359,13 +369,14 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
         cudaMemsetAsync(ix->d_node_pos, 0xff, (size_t)n * sizeof(u32), s);
         cudaMemsetAsync(ix->d_path, 0, (size_t)path_blocks * sizeof(ulonglong2), s);
         cudaMemsetAsync(head, 0, ((size_t)n / 32 + 1) * sizeof(u32), s);
+        cudaMemsetAsync(fork, 0, ((size_t)n / 32 + 1) * sizeof(u32), s);
         cudaMemsetAsync(cnt, 0, sizeof h_cnt, s);
         for (int c = 0; c < 4; c++)
             if (ix->sel_n[c])
                 select_samples_kernel<<<(ix->lpc + 255) / 256, 256, 0, s>>>(
                     ix->d_lines + (u64)c * ix->lpc, ix->lpc, ix->d_sel + ix->sel_off[c], ix->sel_n[c]);
         const StreamView sv = stream_view(ix);
-        succ_kernel<<<blocks, 256, 0, s>>>(sv, succ, head, cnt);
+        succ_kernel<<<blocks, 256, 0, s>>>(sv, succ, head, fork, cnt);
         if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
             break;
         const u32 max_seg = (u32)h_cnt[0];
@@ -384,7 +395,8 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
         const PathArrays pa{ix->d_path_node, ix->d_node_pos, ix->d_path, ix->d_labels, len};
         segment_write_kernel<<<n_seg / 128 + 1, 128, 0, s>>>(sv, k, n_seg, first, succ, off, pa, cnt + 2);
         cycles_kernel<<<blocks, 256, 0, s>>>(sv, k, succ, pa, off + n_seg, cnt + 2);
-        path_letters_kernel<<<(path_blocks + 255) / 256, 256, 0, s>>>(sv, ix->d_path_node, ix->d_path, path_blocks);
+        path_letters_kernel<<<(path_blocks + 255) / 256, 256, 0, s>>>(sv, ix->d_path_node, fork, ix->d_path,
+                                                                         path_blocks);
         node_nibbles_kernel<<<(n / 2 + 1 + 255) / 256, 256, 0, s>>>(n, k, ix->d_labels, len, ix->d_node);
         qbits_kernel<<<blocks, 256, 0, s>>>(n, q, ix->d_labels, len, ix->d_qbits);
         marks_kernel<<<(mark_words + 255) / 256, 256, 0, s>>>(n, ix->d_node, ix->d_marks, mark_words);
@@ -400,6 +412,7 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
         rc = set_error("CUDA error while building the walk's structures: %s", cudaGetErrorString(e));
     cudaFree(succ);
     cudaFree(head);
+    cudaFree(fork);
     cudaFree(first);
     cudaFree(off);
     cudaFree(len);

@@ -131,8 +131,11 @@ struct StreamView {
 //    first successor of path_node[i] unless position i + 1 starts a segment.
 //    node_pos is the inverse.  path[b] holds positions 32 b .. 32 b + 31: x =
 //    the last letters of their labels (MSB-first), y = segment starts (position
-//    32 b + t at bit 63 - t).  A read that follows the graph is compared with a
-//    path 32 letters at a time, and its answers lie in order in path_node.
+//    32 b + t at bit 63 - t) and, at bit 31 - t, the positions that are one or
+//    follow a node with more edges: before the others, the path's letter is the
+//    only one that continues.  A read that follows the graph is compared with a
+//    path 32 letters at a time, and its answers lie in order in path_node.  The
+//    root is a segment of its own.
 struct WalkView {
     const u64 *labels;
     const u32 *qbits;

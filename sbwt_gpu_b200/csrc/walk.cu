@@ -58,10 +58,13 @@ constexpr u32 kPiece = 256;  // k-mers per run at most: reads of 250 letters sta
 constexpr u64 kFillAhead = 8ull << 20;
 
 // What is left of one run: k-mer j (letters from pos on) and `left` k-mers
-// after it.  hint: 0, or 1 + offset of the q-mer to probe first.
+// after it.  hint: 0, or 1 + offset of the q-mer to probe first.  at: 0, or the
+// path position of k-mer j if its letters go on along the path of the stretch
+// found last (after a substituted letter they do).
 template <class IX> struct Run {
     IX pos, j;
-    u32 left, hint;
+    uint16_t left, hint;
+    u32 at;
 };
 
 // Node of a k-mer (first letter at the top, letters past k ignored), or kNoNode.
@@ -108,11 +111,6 @@ __device__ __forceinline__ u64 letters_at(const SearchArgs &a, u64 pos) {
     return (w0 << sh) | (shr_clamp(w1, 63u - sh) >> 1);
 }
 
-__device__ __forceinline__ u32 letter_at(const SearchArgs &a, u64 pos) {
-    pos = min(pos, a.max_pos);
-    return (u32)(__ldg(a.words + (pos >> 5)) >> (62u - 2u * (u32)(pos & 31u))) & 3u;
-}
-
 // Node of the k-mer that follows the k-mer of node v with letter c, or kNoNode.
 __device__ __forceinline__ u32 step(const SearchArgs &a, const LinesRanker &rk, const u32 *C, u32 v, u32 c) {
     const ulonglong4 *lines = rk.lines + (u64)c * rk.lpc;
@@ -127,9 +125,11 @@ __device__ __forceinline__ u32 step(const SearchArgs &a, const LinesRanker &rk, 
 }
 
 // How many of the path's nodes from position i on follow the read's letters from
-// pos on, in the same segment, at most `limit`.
-__device__ __forceinline__ u32 extend(const SearchArgs &a, u32 i, u64 pos, u32 limit) {
+// pos on, in the same segment, at most `limit`.  closed: the letter after them
+// continues no indexed k-mer.
+__device__ __forceinline__ u32 extend(const SearchArgs &a, u32 i, u64 pos, u32 limit, bool &closed) {
     u32 n = 0;
+    closed = false;
     while (n < limit) {
         const u32 sh = (i + n) & 31u;
         const ulonglong2 b = ld_nc2(a.wv.path + ((i + n) >> 5));
@@ -137,9 +137,23 @@ __device__ __forceinline__ u32 extend(const SearchArgs &a, u32 i, u64 pos, u32 l
         const u32 same = min((u32)__clzll((long long)diff) >> 1, 32u - sh);
         const u32 good = min(same, (u32)__clz((int)((u32)(b.y >> 32) << sh)));
         n += good;
-        if (good < 32u - sh) break;
+        if (good < 32u - sh) {
+            closed = n < limit && !((b.y >> (31u - sh - good)) & 1u);
+            break;
+        }
     }
     return min(n, limit);
+}
+
+// Whether path position x is the node of this k-mer: the k path letters up to x are its own and follow each other.
+__device__ __forceinline__ bool on_path(const SearchArgs &a, u32 x, u64 kmer) {
+    const u32 k = a.k;
+    if (x < k - 1u || x >= a.wv.n) return false;
+    const u32 i = x - (k - 1u), sh = i & 31u;
+    const ulonglong2 b0 = ld_nc2(a.wv.path + (i >> 5)), b1 = ld_nc2(a.wv.path + (i >> 5) + 1);
+    const u64 letters = (b0.x << (2u * sh)) | (shr_clamp(b1.x, 63u - 2u * sh) >> 1);
+    const u32 starts = __funnelshift_l((u32)(b1.y >> 32), (u32)(b0.y >> 32), sh);
+    return ((letters ^ kmer) >> (64u - 2u * k)) == 0 && ((starts << 1) >> (33u - k)) == 0;
 }
 
 // 16 letters from pos on (at least the first `need`), the first at the top: from half words of 16 letters, a
@@ -198,7 +212,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
             const IX max_pos = (IX)a.max_pos;
             bool act = false;
             IX pos = 0, J = 0;
-            u32 left = 0;
+            u32 left = 0, at = 0;
             u32 hint = 0;  // ~0: second probe
             for (;;) {
                 if (more && nr < 32u) {
@@ -247,8 +261,8 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                             const u32 from = min(idx * size, o_len), to = min(from + size, o_len);
                             stop = o_b0 + to;
                             const IX j = o_b0 + from;
-                            pool[nr + lane] =
-                                Run<IX>{(IX)((IX)a.row_starts[crow + own] + (j - o_ks)), j, to - from - 1u, 0u};
+                            pool[nr + lane] = Run<IX>{(IX)((IX)a.row_starts[crow + own] + (j - o_ks)), j,
+                                                      (uint16_t)(to - from - 1u), 0, 0};
                         }
                         nr += total;
                         if (total) {
@@ -271,6 +285,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         J = e.j;
                         left = e.left;
                         hint = e.hint;
+                        at = e.at;
                         act = true;
                     }
                     nr -= take;
@@ -301,12 +316,13 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         left -= adv;
                         pos += adv;
                         J += adv;
+                        if (at) at += adv;
                         hint = !second && hint > adv ? hint - adv : 0u;
                     }
                 }
                 if (const u32 pm = __ballot_sync(kFull, pass)) {
                     if (pass) {
-                        pool[kPool - 1u - nw - __popc(pm & lt)] = Run<IX>{pos, J, left, 0u};
+                        pool[kPool - 1u - nw - __popc(pm & lt)] = Run<IX>{pos, J, (uint16_t)left, 0, at};
                         act = false;
                     }
                     nw += __popc(pm);
@@ -314,7 +330,8 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                 if (nw >= kBatch) break;
             }
             const u32 am = __ballot_sync(kFull, act);
-            if (act) pool[nr + __popc(am & lt)] = Run<IX>{pos, J, left, hint == ~0u ? 0u : hint};
+            if (act)
+                pool[nr + __popc(am & lt)] = Run<IX>{pos, J, (uint16_t)left, (uint16_t)(hint == ~0u ? 0u : hint), at};
             nr += __popc(am);
             __syncwarp();
         }
@@ -322,7 +339,9 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
         // ======== walk: look up, step and extend until every run is settled or has to be probed again
         {
             IX pos = 0, J = 0;  // of the next k-mer
-            u32 left = 0, v = kNoNode;  // v: node of k-mer J - 1, or kNoNode: look J up
+            u32 left = 0;
+            u32 v = kNoNode;  // node of k-mer J - 1, or kNoNode: look J up
+            u32 at = 0;       // v == kNoNode: path position to try first
             bool act = false;
             for (;;) {
                 const u32 idle = __ballot_sync(kFull, !act);
@@ -334,24 +353,33 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         J = e.j;
                         left = e.left;
                         v = kNoNode;
+                        at = e.at;
                         act = true;
                     }
                     nw -= take;
                 } else if (idle == kFull) {
                     break;
                 }
-                u32 count = 0, at = 0;  // found k-mers from J on, the first one's path position
-                bool known = false;
+                u32 count = 0;     // found k-mers from J on, the first one at path position `at`
+                bool miss = false; // the k-mer after those is absent: the rest goes back to be probed
+                u32 hint = 0;
                 if (act) {
-                    known = v != kNoNode;
-                    v = known ? step(a, rk, sC, v, letter_at(a, (u64)pos + (k - 1u)))
-                              : lookup(a, letters_at(a, pos));
+                    const u64 kmer = letters_at(a, pos);
                     if (v != kNoNode) {
-                        at = __ldg(a.wv.node_pos + v);
-                        count = 1u + extend(a, at + 1u, (u64)pos + k, left);
+                        v = step(a, rk, sC, v, (u32)(kmer >> (64u - 2u * k)) & 3u);
+                        if (v == kNoNode) hint = k - 1u;  // the letter of the missing edge, at offset k - 2 of k-mer J + 1
+                        else at = __ldg(a.wv.node_pos + v);
+                    } else if (!at || !on_path(a, at, kmer)) {
+                        v = lookup(a, kmer);
+                        at = v != kNoNode ? __ldg(a.wv.node_pos + v) : 0u;
+                    } else {
+                        v = ~0u;  // found
                     }
+                    bool closed = false;
+                    if (v != kNoNode) count = 1u + extend(a, at + 1u, (u64)pos + k, left, closed);
+                    miss = v == kNoNode || closed;
+                    if (closed) hint = k - 1u;
                 }
-                const bool miss = act && count == 0;  // k-mer J is absent: those after it go back to be probed
                 if (a.answers) {
                     for (u32 m = __ballot_sync(kFull, count != 0); m; m &= m - 1u) {
                         const int src = __ffs(m) - 1;
@@ -362,22 +390,21 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                             if (t < c) out[t] = (u64)__ldg(a.wv.path_node + f + t);
                     }
                 }
-                if (miss) {
-                    act = false;
-                    pos++;
-                    J++;
-                } else if (count) {
-                    if (a.member) set_bits(a.member, J, count);
-                    act = count <= left;
-                    left -= count;
-                    pos += count;
-                    J += count;
-                    if (act) v = __ldg(a.wv.path_node + at + count - 1u);
+                bool back = false;
+                if (act) {
+                    if (count && a.member) set_bits(a.member, J, count);
+                    const u32 adv = count + (miss ? 1u : 0u);  // settled from J on, at most left + 1
+                    act = adv <= left;
+                    back = act && miss;
+                    if (act && !miss) v = __ldg(a.wv.path_node + at + count - 1u);
+                    if (at) at += adv;  // where k-mer J + adv lies if the read goes on along this path
+                    left -= adv;
+                    pos += adv;
+                    J += adv;
+                    act = act && !miss;
                 }
-                const bool back = miss && left != 0;
                 const u32 bm = __ballot_sync(kFull, back);
-                // hint: the letter of a missing edge, at offset k - 2 of the next k-mer
-                if (back) pool[nr + __popc(bm & lt)] = Run<IX>{pos, J, left - 1u, known ? k - 1u : 0u};
+                if (back) pool[nr + __popc(bm & lt)] = Run<IX>{pos, J, (uint16_t)left, (uint16_t)hint, at};
                 nr += __popc(bm);
                 __syncwarp();
             }
@@ -389,21 +416,29 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
 
 namespace {
 
-// answers[0 .. n) = absent, 32 bytes a thread and iteration where they are aligned.  Ahead of the walk, at the
-// rate of a plain fill; written by the walk as it settles absent k-mers, the same bytes pushed the q-mer bitmap out
-// of L2 (it then missed at every probe) and did not overlap with the probing: 1.2G k-mers, nine tenths of the reads
-// foreign, 100M columns: 4.18 ms a call against 4.85 (and 4.18 against 4.94 with each warp filling its chunk first).
-__global__ void __launch_bounds__(512) fill_kernel(u64 *__restrict__ answers, u64 n, const u64 *runs_dev,
-                                                   const u64 *__restrict__ kstart, u64 n_rows) {
+// answers[0 .. n) = absent, ahead of the walk.  Written by the walk as it settles absent k-mers, the same bytes
+// pushed the q-mer bitmap out of L2 (it then missed at every probe) and did not overlap with the probing: 1.2G
+// k-mers, nine tenths of the reads foreign, 100M columns: 4.18 ms a call against 4.85 (4.94 with each warp filling
+// its chunk first).  Four 32-byte stores a thread, blocks in order: 7.6 TB/s for 9.6 GB; a grid-stride loop of as many
+// threads as the device holds 6.3.
+constexpr u32 kFillThreads = 512, kFillStores = 4;
+__global__ void __launch_bounds__(kFillThreads) fill_kernel(u64 *__restrict__ answers, u64 n, const u64 *runs_dev,
+                                                            const u64 *__restrict__ kstart, u64 n_rows) {
     if (runs_dev && !runs_usable(*runs_dev, n)) return;  // the answers still hold the positions of the per-k-mer search
     if (!runs_dev) n = min(n, kstart[n_rows]);
     const u64 head = min(n, (u64)((32u - (reinterpret_cast<uintptr_t>(answers) & 31u)) & 31u) / 8u);
-    const u64 t0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
-    const u64 quads = (n - head) / 4u;
-    for (u64 t = t0; t < quads; t += step)
-        asm volatile("st.global.v4.u64 [%0], {%1, %1, %1, %1};" ::"l"(answers + head + 4u * t), "l"(~0ull) : "memory");
-    if (t0 < head) answers[t0] = ~0ull;
-    if (t0 < n - head - 4u * quads) answers[head + 4u * quads + t0] = ~0ull;
+    const u64 quads = (n - head) / 4u, tail = n - head - 4u * quads;
+    const u64 b = (u64)blockIdx.x * (kFillThreads * kFillStores) + threadIdx.x;
+#pragma unroll
+    for (u32 i = 0; i < kFillStores; i++) {
+        const u64 t = b + i * kFillThreads;
+        if (t < quads)
+            asm volatile("st.global.v4.u64 [%0], {%1, %1, %1, %1};" ::"l"(answers + head + 4u * t), "l"(~0ull) : "memory");
+    }
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < head) answers[threadIdx.x] = ~0ull;
+        if (threadIdx.x < tail) answers[head + 4u * quads + threadIdx.x] = ~0ull;
+    }
 }
 
 }  // namespace
@@ -432,7 +467,8 @@ int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *b
     if (blocks_out) *blocks_out = blocks;
     SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
     if (a.answers && a.n_kmers >= kFillAhead) {
-        fill_kernel<<<(unsigned)ix->num_sms * 4u, 512, 0, s>>>(a.answers, a.n_kmers, a.runs_dev, a.kstart, a.n_rows);
+        const u64 per = 4ull * kFillThreads * kFillStores;
+        fill_kernel<<<(unsigned)((a.n_kmers + per - 1) / per), kFillThreads, 0, s>>>(a.answers, a.n_kmers, a.runs_dev, a.kstart, a.n_rows);
         SBWT_CHECK_CUDA(cudaGetLastError());
     }
     return launch_kernel(kern, blocks, kWarps * 32, s, ix, LinesRanker{ix->d_lines, ix->lpc}, a);
