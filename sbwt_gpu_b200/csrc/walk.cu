@@ -317,7 +317,9 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         pos += adv;
                         J += adv;
                         if (at) at += adv;
-                        hint = !second && hint > adv ? hint - adv : 0u;
+                        const bool ahead = !second && hint;  // the letter that ended a found stretch lies in k-mer J
+                        hint = ahead && hint > adv ? hint - adv : 0u;
+                        pass = ahead && !hint && at;  // behind it the read most likely goes on along its path
                     }
                 }
                 if (const u32 pm = __ballot_sync(kFull, pass)) {
