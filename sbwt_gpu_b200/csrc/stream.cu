@@ -40,10 +40,14 @@ __global__ void select_samples_kernel(const ulonglong4 *__restrict__ lines, u32 
 
 // ---- paths: each column's first outgoing edge links it to one successor (the
 // root's none: it has no letter), and every node but the root has one incoming
-// edge, so the links form chains and cycles.  They are cut into segments at the nodes without a link to them and at
-// one node in kSegment (by a hash), so that one thread per segment walks it: once
-// to size it, once to write it together with the labels, which roll along the
-// segment from its first node's (k select steps back).
+// edge, so the links form chains and cycles.  They are cut into segments at the
+// nodes without a link to them and at one node in kSegment (by a hash), so that
+// one thread per segment walks it: once to size it, once to write it together
+// with the labels, which roll along the segment from its first node's (k select
+// steps back).  In between the segments are put in order by pointer doubling, so
+// that those of one chain adjoin and a read runs on over the cuts: with every cut
+// a path's end, a quarter of the stretches of 150-letter reads ended there and
+// took a rank step each.
 
 constexpr u32 kSegment = 256;
 
@@ -91,19 +95,69 @@ __global__ void heads_kernel(u32 n, const u32 *__restrict__ head, u32 *__restric
     if (is) first[base + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u))] = v;
 }
 
-__global__ void segment_len_kernel(u32 n_seg, const u32 *__restrict__ first, const u32 *__restrict__ succ,
-                                   u32 *__restrict__ len) {
+constexpr u32 kNoSeg = ~0u;
+
+// pos[first node of segment i] = i, for the links between segments
+__global__ void segment_ids_kernel(u32 n_seg, const u32 *__restrict__ first, u32 *__restrict__ pos,
+                                   u32 *__restrict__ prev) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n_seg) return;
-    u32 l = 0;
-    if (i < n_seg) {
-        u32 v = first[i];
-        do {
-            v = succ[v];
-            l++;
-        } while (v && !cut_here(v));
+    if (i >= n_seg) return;
+    pos[first[i]] = i;
+    prev[i] = kNoSeg;
+}
+
+__global__ void segment_len_kernel(u32 n_seg, const u32 *__restrict__ first, const u32 *__restrict__ succ,
+                                   const u32 *__restrict__ pos, u32 *__restrict__ len, u32 *__restrict__ prev) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_seg) return;
+    u32 l = 0, v = first[i];
+    do {
+        v = succ[v];
+        l++;
+    } while (v && !cut_here(v));
+    len[i] = l;
+    if (v) prev[pos[v]] = i;
+}
+
+// Per segment i: before = nodes of the segments between i and ptr (both
+// excluded), head = the farthest of them (i if there is none), low = the
+// smallest of i and them.
+struct SegRank {
+    u32 ptr, before, head, low;
+};
+
+__global__ void rank_init_kernel(u32 n_seg, const u32 *__restrict__ prev, SegRank *__restrict__ r) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_seg) r[i] = SegRank{prev[i], 0u, i, i};
+}
+
+// One doubling round.
+__global__ void rank_double_kernel(u32 n_seg, const u32 *__restrict__ len, const SegRank *__restrict__ r,
+                                   SegRank *__restrict__ out) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_seg) return;
+    SegRank x = r[i];
+    if (x.ptr != kNoSeg) {
+        const SegRank y = r[x.ptr];
+        x = SegRank{y.ptr, x.before + len[x.ptr] + y.before, y.head, min(x.low, y.low)};
     }
-    len[i] = l;  // len[n_seg] = 0: its prefix sum is the number of nodes reached
+    out[i] = x;
+}
+
+// After all rounds a segment that still has a ptr lies on a cycle: the smallest of each becomes its first.
+__global__ void open_cycles_kernel(u32 n_seg, const SegRank *__restrict__ r, u32 *__restrict__ prev,
+                                   unsigned long long *__restrict__ opened) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_seg || r[i].ptr == kNoSeg || r[i].low != i) return;
+    prev[i] = kNoSeg;
+    atomicAdd(opened, 1ull);
+}
+
+// total[first segment of a chain] = nodes of the chain (0 for the other segments, and at n_seg).
+__global__ void chain_len_kernel(u32 n_seg, const SegRank *__restrict__ r, const u32 *__restrict__ len,
+                                 u32 *__restrict__ total) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_seg) atomicMax(total + r[i].head, r[i].before + len[i]);
 }
 
 struct PathArrays {
@@ -113,8 +167,9 @@ struct PathArrays {
     uint8_t *len;       // letters of the label before its $ padding, at most k
 };
 
-// The segment of `count` nodes that starts at v goes to positions off .. off + count - 1.
-__device__ void write_segment(const StreamView &sv, u32 k, const u32 *succ, u32 v, u32 off, u32 count,
+// The segment of `count` nodes that starts at v goes to positions off .. off + count - 1; starts: no other one
+// leads into it.
+__device__ void write_segment(const StreamView &sv, u32 k, const u32 *succ, u32 v, u32 off, u32 count, bool starts,
                               const PathArrays &a, unsigned long long *bad) {
     const u64 mask = k < 32u ? (1ull << (2u * k)) - 1ull : ~0ull;
     u64 code = 0;
@@ -127,7 +182,7 @@ __device__ void write_segment(const StreamView &sv, u32 k, const u32 *succ, u32 
             u = 0;
         }
     }
-    atomicOr((unsigned long long *)&a.path[off >> 5].y, 1ull << (63u - (off & 31u)));
+    if (starts) atomicOr((unsigned long long *)&a.path[off >> 5].y, 1ull << (63u - (off & 31u)));
     for (u32 i = 0; i < count; i++) {
         a.node[off + i] = v;
         a.pos[v] = off + i;
@@ -140,10 +195,13 @@ __device__ void write_segment(const StreamView &sv, u32 k, const u32 *succ, u32 
 }
 
 __global__ void segment_write_kernel(const StreamView sv, u32 k, u32 n_seg, const u32 *__restrict__ first,
-                                     const u32 *__restrict__ succ, const u32 *__restrict__ off, const PathArrays a,
-                                     unsigned long long *__restrict__ bad) {
+                                     const u32 *__restrict__ succ, const u32 *__restrict__ len,
+                                     const SegRank *__restrict__ r, const u32 *__restrict__ chain_off,
+                                     const PathArrays a, unsigned long long *__restrict__ bad) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_seg) write_segment(sv, k, succ, first[i], off[i], off[i + 1u] - off[i], a, bad);
+    if (i >= n_seg) return;
+    const SegRank x = r[i];
+    write_segment(sv, k, succ, first[i], chain_off[x.head] + x.before, len[i], x.head == i, a, bad);
 }
 
 // Cycles that no cut falls on (short ones): the thread of a cycle's smallest node writes it.
@@ -153,7 +211,7 @@ __global__ void cycles_kernel(const StreamView sv, u32 k, const u32 *__restrict_
     if (v >= sv.n || *(volatile u32 *)(a.pos + v) != ~0u) return;
     u32 x = succ[v], count = 1;
     for (; x > v; x = succ[x]) count++;
-    if (x == v) write_segment(sv, k, succ, v, atomicAdd(reached, count), count, a, bad);
+    if (x == v) write_segment(sv, k, succ, v, atomicAdd(reached, count), count, true, a, bad);
 }
 
 // The last letters of the path's nodes, 32 positions a thread, and the positions that cannot be judged by the
@@ -341,11 +399,13 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
     const size_t qwords = std::max<size_t>(1, (size_t)((1ull << (2u * q)) / 32u));
     const u32 blocks = (n + 255) / 256;
     // scratch: first successors, head bits, label lengths, segments; counters: segments (upper bound),
-    // segments, nodes without a predecessor, columns the forward walk cannot take
+    // segments, nodes without a predecessor, columns the forward walk cannot take, cycles of segments
     u32 *succ = nullptr, *head = nullptr, *fork = nullptr, *first = nullptr, *off = nullptr;
+    u32 *seg_len = nullptr, *prev = nullptr;
+    SegRank *rank[2] = {nullptr, nullptr};
     uint8_t *len = nullptr;
     void *tmp = nullptr;
-    unsigned long long *cnt = nullptr, h_cnt[4] = {0, 0, 0, 0};
+    unsigned long long *cnt = nullptr, h_cnt[5] = {0, 0, 0, 0, 0};
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
@@ -366,7 +426,6 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
             break;
         cudaMemsetAsync(ix->d_sel, 0, total * sizeof(u32), s);
         cudaMemsetAsync(ix->d_qbits, 0, qwords * sizeof(u32), s);
-        cudaMemsetAsync(ix->d_node_pos, 0xff, (size_t)n * sizeof(u32), s);
         cudaMemsetAsync(ix->d_path, 0, (size_t)path_blocks * sizeof(ulonglong2), s);
         cudaMemsetAsync(head, 0, ((size_t)n / 32 + 1) * sizeof(u32), s);
         cudaMemsetAsync(fork, 0, ((size_t)n / 32 + 1) * sizeof(u32), s);
@@ -380,20 +439,40 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
         if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
             break;
         const u32 max_seg = (u32)h_cnt[0];
-        if (!ok(cudaMalloc(&first, (size_t)max_seg * sizeof(u32))) || !ok(cudaMalloc(&off, ((size_t)max_seg + 1) * sizeof(u32))))
+        if (!ok(cudaMalloc(&first, (size_t)max_seg * sizeof(u32))) ||
+            !ok(cudaMalloc(&off, ((size_t)max_seg + 1) * sizeof(u32))) ||
+            !ok(cudaMalloc(&seg_len, (size_t)max_seg * sizeof(u32))) || !ok(cudaMalloc(&prev, (size_t)max_seg * sizeof(u32))) ||
+            !ok(cudaMalloc(&rank[0], (size_t)max_seg * sizeof(SegRank))) ||
+            !ok(cudaMalloc(&rank[1], (size_t)max_seg * sizeof(SegRank))))
             break;
         heads_kernel<<<blocks, 256, 0, s>>>(n, head, first, cnt + 1);
         if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
             break;
-        const u32 n_seg = (u32)h_cnt[1];
-        segment_len_kernel<<<n_seg / 128 + 1, 128, 0, s>>>(n_seg, first, succ, off);
+        const u32 n_seg = (u32)h_cnt[1], seg_blocks = (n_seg + 127) / 128;
+        segment_ids_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, first, ix->d_node_pos, prev);
+        segment_len_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, first, succ, ix->d_node_pos, seg_len, prev);
+        int cur = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            rank_init_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, prev, rank[cur]);
+            for (u64 reach = 1; reach < 2ull * n_seg; reach *= 2, cur ^= 1)
+                rank_double_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, seg_len, rank[cur], rank[cur ^ 1]);
+            if (pass) break;
+            open_cycles_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, rank[cur], prev, cnt + 4);
+            if (!ok(cudaMemcpyAsync(h_cnt, cnt, sizeof h_cnt, cudaMemcpyDeviceToHost, s)) || !ok(cudaStreamSynchronize(s)))
+                break;
+            if (h_cnt[4] == 0) break;
+        }
+        if (e != cudaSuccess) break;
+        cudaMemsetAsync(off, 0, ((size_t)n_seg + 1) * sizeof(u32), s);
+        chain_len_kernel<<<seg_blocks, 128, 0, s>>>(n_seg, rank[cur], seg_len, off);
         size_t tmp_bytes = 0;
         if (!ok(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, off, off, (int64_t)n_seg + 1, s)) ||
             !ok(cudaMalloc(&tmp, tmp_bytes ? tmp_bytes : 1)) ||
-            !ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, off, off, (int64_t)n_seg + 1, s)))
+            !ok(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, off, off, (int64_t)n_seg + 1, s)) ||
+            !ok(cudaMemsetAsync(ix->d_node_pos, 0xff, (size_t)n * sizeof(u32), s)))
             break;
         const PathArrays pa{ix->d_path_node, ix->d_node_pos, ix->d_path, ix->d_labels, len};
-        segment_write_kernel<<<n_seg / 128 + 1, 128, 0, s>>>(sv, k, n_seg, first, succ, off, pa, cnt + 2);
+        segment_write_kernel<<<seg_blocks, 128, 0, s>>>(sv, k, n_seg, first, succ, seg_len, rank[cur], off, pa, cnt + 2);
         cycles_kernel<<<blocks, 256, 0, s>>>(sv, k, succ, pa, off + n_seg, cnt + 2);
         path_letters_kernel<<<(path_blocks + 255) / 256, 256, 0, s>>>(sv, ix->d_path_node, fork, ix->d_path,
                                                                          path_blocks);
@@ -415,6 +494,10 @@ int build_stream(sbwt_index *ix, cudaStream_t s) {
     cudaFree(fork);
     cudaFree(first);
     cudaFree(off);
+    cudaFree(seg_len);
+    cudaFree(prev);
+    cudaFree(rank[0]);
+    cudaFree(rank[1]);
     cudaFree(len);
     cudaFree(tmp);
     cudaFree(cnt);
