@@ -537,7 +537,7 @@ void set_gather_policies(const sbwt_index *ix, SearchArgs &a) {
     const u64 half = ix->l2_bytes / 2;
     const u64 pre_bytes = ix->p ? (1ull << (2 * ix->p)) * (ix->pre64 ? 16ull : 8ull) : 0;
     const int ev = ix->shape.evict;
-    a.ef_pre = a.runs && ev != 1 && (ev == 2 || pre_bytes > half);
+    a.ef_pre = (a.runs || a.walk) && ev != 1 && (ev == 2 || pre_bytes > half);
 }
 
 SearchArgs base_args(const sbwt_index *ix, bool rows, u64 n_kmers, bool filtered) {
@@ -558,13 +558,13 @@ SearchArgs base_args(const sbwt_index *ix, bool rows, u64 n_kmers, bool filtered
     a.chunk = search_chunk(ix, rows);
     a.runs = rows && runs_form(ix);
     a.stream = a.runs && filtered && stream_form(ix);
-    a.walk = a.runs && !filtered && stream_form(ix);
+    a.walk = !filtered && stream_form(ix);
     a.index64 = (u32)ix->shape.index64;
     a.pre32 = a.runs ? ix->d_pre32 : nullptr;
     if (a.stream || a.walk) a.sv = stream_view(ix);
     if (a.walk) {
         a.wv = walk_view(ix);
-        a.chunk = walk_chunk(ix, n_kmers);
+        if (rows) a.chunk = walk_chunk(ix, n_kmers);
     }
     set_gather_policies(ix, a);
     return a;

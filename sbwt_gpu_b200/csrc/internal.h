@@ -50,7 +50,8 @@ struct SearchArgs {
     u32 index64;                  // with `runs`: the walk's 64-bit index form whatever the batch size
     u32 ef_pre;                   // with `runs`: evict-first gathers from the presearch table (set when
                                   // it cannot stay in L2; device.cuh)
-    u32 walk;                     // read mode: the forward walk (walk.cu), with wv and sv
+    u32 walk;                     // the searches of walk.cu, with wv and sv: the forward walk in read mode, else
+                                  // the list search
     dev::StreamView sv;           // node nibbles, select samples (stream.cuh)
     dev::WalkView wv;             // labels, q-mer bitmap, group marks (stream.cuh)
     uint32_t *member;             // with `runs`: membership bitmap written by the search kernel, or NULL
@@ -270,5 +271,6 @@ bool run32_ok(const SearchArgs &a);
 // walk.cu
 u32 walk_chunk(const sbwt_index *ix, u64 n_kmers);
 int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *launched_blocks);
+int launch_list(const sbwt_index *ix, SearchArgs &a, cudaStream_t s);
 
 }  // namespace sbwt

@@ -852,7 +852,7 @@ u32 search_chunk(const sbwt_index *ix, bool rows) {
 int launch_search(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *blocks) {
     const KernelShape &sh = ix->shape;
     if (a.n_kmers == 0) return 0;
-    if (a.walk) return launch_walk(ix, a, s, blocks);
+    if (a.walk) return a.positions || a.kmer_list ? launch_list(ix, a, s) : launch_walk(ix, a, s, blocks);
     if (a.reject && !(a.runs && sh.layout == SBWT_LAYOUT_LINES && sh.tpk == 1 && sh.kpt == 0))
         return set_error("the prefiltered search of reads needs the run walk on the line layout "
                          "(search mode stream or skip, one lane per k-mer, queue-fed)");

@@ -35,6 +35,7 @@
 #include "device.cuh"
 #include "internal.h"
 #include "launch.cuh"
+#include "mlp_kernels.cuh"
 #include "rank.cuh"
 #include "stream.cuh"
 
@@ -58,9 +59,9 @@ constexpr u32 kPiece = 256;  // k-mers per run at most: reads of 250 letters sta
 constexpr u64 kFillAhead = 8ull << 20;
 
 // What is left of one run: k-mer j (letters from pos on) and `left` k-mers
-// after it.  hint: 0, or 1 + offset of the q-mer to probe first.  at: 0, or the
-// path position of k-mer j if its letters go on along the path of the stretch
-// found last (after a substituted letter they do).
+// after it.  hint: 0, or 1 + offset in k-mer j of the letter that ended the
+// stretch found last.  at: 0, or the path position of k-mer j if its letters go
+// on along the path of that stretch (after a substituted letter they do).
 template <class IX> struct Run {
     IX pos, j;
     uint16_t left, hint;
@@ -212,8 +213,8 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
             const IX max_pos = (IX)a.max_pos;
             bool act = false;
             IX pos = 0, J = 0;
-            u32 left = 0, at = 0;
-            u32 hint = 0;  // ~0: second probe
+            u32 left = 0, at = 0, hint = 0;
+            u32 tries = 0;  // pairs of q-mers of k-mer J found present
             for (;;) {
                 if (more && nr < 32u) {
                     if (cj >= ce) {
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         left = e.left;
                         hint = e.hint;
                         at = e.at;
+                        tries = 0;
                         act = true;
                     }
                     nr -= take;
@@ -297,8 +299,10 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                 // ---- one round: q-mers at offsets o and o - d of the current k-mer
                 bool pass = false;
                 if (act) {
-                    const bool second = hint == ~0u;
-                    const u32 o = second ? o_max / 2u : hint ? min(hint - 1u, o_max) : o_max;
+                    // the letter that ended a stretch is in no indexed k-mer after those before it: the q-mers that
+                    // hold it are probed from the right one on; otherwise the right end, then the middle
+                    const u32 last = hint ? min(hint - 1u, o_max) : o_max;
+                    const u32 o = hint ? last - 2u * tries : tries ? o_max / 2u : o_max;
                     const u32 d = o ? two : 0u;
                     const u32 x = half_words(a, min(pos + (o - d), max_pos), a.wv.q + d);
                     u32 adv = o + 1u;
@@ -308,8 +312,8 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         adv -= d;
                     }
                     if (in) {
-                        pass = second;
-                        hint = ~0u;
+                        tries++;
+                        pass = tries == 2u || (hint && (o < 2u || o + a.wv.q < hint + 2u));
                     } else if (adv > left) {
                         act = false;
                     } else {
@@ -317,14 +321,14 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         pos += adv;
                         J += adv;
                         if (at) at += adv;
-                        const bool ahead = !second && hint;  // the letter that ended a found stretch lies in k-mer J
-                        hint = ahead && hint > adv ? hint - adv : 0u;
-                        pass = ahead && !hint && at;  // behind it the read most likely goes on along its path
+                        pass = hint && hint <= adv && at;  // behind that letter the read most likely goes on along its path
+                        hint = hint > adv ? hint - adv : 0u;
+                        tries = 0;
                     }
                 }
                 if (const u32 pm = __ballot_sync(kFull, pass)) {
                     if (pass) {
-                        pool[kPool - 1u - nw - __popc(pm & lt)] = Run<IX>{pos, J, (uint16_t)left, 0, at};
+                        pool[kPool - 1u - nw - __popc(pm & lt)] = Run<IX>{pos, J, (uint16_t)left, (uint16_t)hint, at};
                         act = false;
                     }
                     nw += __popc(pm);
@@ -332,8 +336,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                 if (nw >= kBatch) break;
             }
             const u32 am = __ballot_sync(kFull, act);
-            if (act)
-                pool[nr + __popc(am & lt)] = Run<IX>{pos, J, (uint16_t)left, (uint16_t)(hint == ~0u ? 0u : hint), at};
+            if (act) pool[nr + __popc(am & lt)] = Run<IX>{pos, J, (uint16_t)left, (uint16_t)hint, at};
             nr += __popc(am);
             __syncwarp();
         }
@@ -343,7 +346,8 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
             IX pos = 0, J = 0;  // of the next k-mer
             u32 left = 0;
             u32 v = kNoNode;  // node of k-mer J - 1, or kNoNode: look J up
-            u32 at = 0;       // v == kNoNode: path position to try first
+            u32 at = 0;       // v == kNoNode: path position to try first, unless hint says that k-mer J left the path
+            u32 hint = 0;
             bool act = false;
             for (;;) {
                 const u32 idle = __ballot_sync(kFull, !act);
@@ -356,6 +360,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                         left = e.left;
                         v = kNoNode;
                         at = e.at;
+                        hint = e.hint;
                         act = true;
                     }
                     nw -= take;
@@ -364,23 +369,26 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                 }
                 u32 count = 0;     // found k-mers from J on, the first one at path position `at`
                 bool miss = false; // the k-mer after those is absent: the rest goes back to be probed
-                u32 hint = 0;
                 if (act) {
                     const u64 kmer = letters_at(a, pos);
+                    const u32 was = hint;
+                    hint = 0;
                     if (v != kNoNode) {
                         v = step(a, rk, sC, v, (u32)(kmer >> (64u - 2u * k)) & 3u);
-                        if (v == kNoNode) hint = k - 1u;  // the letter of the missing edge, at offset k - 2 of k-mer J + 1
+                        if (v == kNoNode) hint = k;  // the letter of the missing edge
                         else at = __ldg(a.wv.node_pos + v);
-                    } else if (!at || !on_path(a, at, kmer)) {
+                    } else if (was || !at || !on_path(a, at, kmer)) {
                         v = lookup(a, kmer);
-                        at = v != kNoNode ? __ldg(a.wv.node_pos + v) : 0u;
+                        if (v == kNoNode) hint = was;
+                        if (!was) at = 0;
+                        if (v != kNoNode) at = __ldg(a.wv.node_pos + v);
                     } else {
                         v = ~0u;  // found
                     }
                     bool closed = false;
                     if (v != kNoNode) count = 1u + extend(a, at + 1u, (u64)pos + k, left, closed);
                     miss = v == kNoNode || closed;
-                    if (closed) hint = k - 1u;
+                    if (closed) hint = k;
                 }
                 if (a.answers) {
                     for (u32 m = __ballot_sync(kFull, count != 0); m; m &= m - 1u) {
@@ -400,6 +408,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                     back = act && miss;
                     if (act && !miss) v = __ldg(a.wv.path_node + at + count - 1u);
                     if (at) at += adv;  // where k-mer J + adv lies if the read goes on along this path
+                    if (hint) hint--;   // k-mer J + adv is the one after the absent one
                     left -= adv;
                     pos += adv;
                     J += adv;
@@ -417,6 +426,86 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
 }  // namespace
 
 namespace {
+
+// ---------------------------------------------------- lists of k-mers
+//
+// K-mers without neighbours (a list, or the positions of the kernel contract
+// that form no runs): each is probed for q-mers that no indexed k-mer contains,
+// at its two ends, and looked up if both are present.  The probes of kListSlots
+// k-mers a lane overlap; those that pass are collected per warp and looked up 32
+// at a time, so that the few present ones do not idle the other lanes.
+constexpr u32 kListSlots = 4;
+constexpr u32 kListPool = 32 * kListSlots + 31;
+
+__global__ void __launch_bounds__(kWarps * 32, 10) list_kernel(const SearchArgs a) {
+    if (a.runs_dev && runs_usable(*a.runs_dev, a.n_kmers)) return;  // the run walk takes this kernel-contract call
+    struct Item {
+        u64 kmer, j;
+    };
+    __shared__ Item pools[kWarps][kListPool];
+    const u32 lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const u32 lt = (1u << lane) - 1u;
+    const u32 q = a.wv.q, o_max = a.k - q;
+    const mlp::Bloom bloom{a.bloom_bits, a.bloom_mask, a.bloom_hashes};
+    Item *const pool = pools[warp];
+    const u64 step = (u64)gridDim.x * kWarps * (32u * kListSlots);
+    u64 base = ((u64)blockIdx.x * kWarps + warp) * (32u * kListSlots);
+    u32 np = 0;
+    for (;;) {
+        const bool more = base < a.n_kmers;
+        if (more) {
+            u64 km[kListSlots];
+            bool in[kListSlots];
+            u32 n_skip = 0;
+#pragma unroll
+            for (u32 u = 0; u < kListSlots; u++) {
+                const u64 j = base + u * 32u + lane;
+                in[u] = j < a.n_kmers;
+                km[u] = 0;
+                if (in[u]) km[u] = a.kmer_list ? __ldg(a.kmer_list + j) : letters_at(a, a.positions[j]);
+            }
+            if (a.logits) {  // learned-Bloom sandwich: answered "absent" only if both reject
+#pragma unroll
+                for (u32 u = 0; u < kListSlots; u++) {
+                    const u64 j = base + u * 32u + lane;
+                    if (in[u] && __ldg(a.logits + j) < a.tau && !bloom.probe(mlp::kmer_key(km[u], a.k))) {
+                        in[u] = false;
+                        n_skip++;
+                    }
+                }
+                n_skip = __reduce_add_sync(kFull, n_skip);
+                if (a.skipped && lane == 0 && n_skip) atomicAdd(a.skipped, (unsigned long long)n_skip);
+            }
+#pragma unroll
+            for (u32 u = 0; u < kListSlots; u++)
+                if (in[u]) in[u] = q_present(a, (u32)(km[u] >> (64u - 2u * q)));
+#pragma unroll
+            for (u32 u = 0; u < kListSlots; u++)
+                if (in[u]) in[u] = q_present(a, (u32)((km[u] << (2u * o_max)) >> (64u - 2u * q)));
+#pragma unroll
+            for (u32 u = 0; u < kListSlots; u++) {
+                const u64 j = base + u * 32u + lane;
+                const u32 m = __ballot_sync(kFull, in[u]);
+                if (in[u]) pool[np + __popc(m & lt)] = Item{km[u], j};
+                else if (j < a.n_kmers) a.answers[j] = ~0ull;
+                np += __popc(m);
+            }
+            base += step;
+            __syncwarp();
+        }
+        while (np >= 32u || (np && !more)) {
+            const u32 take = min(np, 32u);
+            np -= take;
+            if (lane < take) {
+                const Item it = pool[np + lane];
+                const u32 v = lookup(a, it.kmer);
+                a.answers[it.j] = v != kNoNode ? (u64)v : ~0ull;
+            }
+        }
+        __syncwarp();
+        if (!more) break;
+    }
+}
 
 // answers[0 .. n) = absent, ahead of the walk.  Written by the walk as it settles absent k-mers, the same bytes
 // pushed the q-mer bitmap out of L2 (it then missed at every probe) and did not overlap with the probing: 1.2G
@@ -454,6 +543,16 @@ u32 walk_chunk(const sbwt_index *ix, u64 n_kmers) {
     u32 c = 32u;
     while (c < top && (u64)c * warps < n_kmers) c *= 2u;
     return c;
+}
+
+int launch_list(const sbwt_index *ix, SearchArgs &a, cudaStream_t s) {
+    int per_sm = 0;
+    SBWT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, list_kernel, kWarps * 32, 0));
+    const u64 per = (u64)kWarps * 32u * kListSlots, need = (a.n_kmers + per - 1) / per;
+    const u32 blocks = (u32)std::min<u64>((u64)std::max(per_sm, 1) * (u64)ix->num_sms, need);
+    list_kernel<<<blocks, kWarps * 32, 0, s>>>(a);
+    SBWT_CHECK_CUDA(cudaGetLastError());
+    return 0;
 }
 
 int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *blocks_out) {

@@ -94,3 +94,40 @@ def test_another_k_than_the_index(cuda, dk):
         got = _search(ix, letters, rows, nk)
         ix.set_search_mode(sg.SEARCH_EVERY_KMER)
         assert np.array_equal(got, _search(ix, letters, rows, nk))
+
+
+@pytest.mark.parametrize("k,p", [(4, 2), (16, 8), (31, 10), (32, 12)])
+def test_kmer_lists_equal_the_oracle(cuda, k, p):
+    """Lists of single k-mers on both sides of a warp's and a block's share, and positions without runs."""
+    import torch
+    rng = wl.rng_for(2000 + k)
+    seqs = _seqs("ties", k, rng) + _seqs("branches", k, rng)
+    built = sg.build_sbwt([s.encode() for s in seqs], k)
+    text = "".join(seqs)
+    at = rng.integers(0, len(text) - k + 1, size=3000)
+    parts = [text[i:i + k] for i in at]
+    parts[::3] = [wl.random_bases(rng, k).tobytes().decode() for _ in parts[::3]]
+    letters, rows = _rows(parts)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, p)
+    codes = np.searchsorted(wl.ACGT, letters).reshape(-1, k).astype(np.uint64)
+    words = np.zeros(len(parts), dtype=np.uint64)
+    for i in range(k):
+        words |= codes[:, i] << np.uint64(62 - 2 * i)
+    junk = rng.integers(0, 2**63, size=words.size, dtype=np.int64).astype(np.uint64)
+    if k < 32:
+        words |= junk & np.uint64((1 << (64 - 2 * k)) - 1)  # letters past the k-mer do not count
+    d_words = torch.from_numpy(words.view(np.int64)).cuda()
+    packed = torch.from_numpy(wl.pack_words(np.frombuffer((text + "A" * 32).encode(), dtype=np.uint8)).view(np.int64)).cuda()
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        for n in (1, 31, 32, 33, 127, 128, 129, 511, 513, 3000):
+            ans = torch.full((n + 1,), -7, dtype=torch.int64, device="cuda")
+            ix.search_kmers(d_words, ans, n)
+            torch.cuda.synchronize()
+            got = ans.cpu().numpy().view(np.uint64)
+            assert np.array_equal(got[:n], want[:n]) and got[n] == np.uint64(2**64 - 7)
+        pos = torch.from_numpy(at.astype(np.int64)).cuda()  # random positions: no runs
+        ix.search_packed(packed, pos, pos.numel())
+        torch.cuda.synchronize()
+        l2, r2 = _rows([text[i:i + k] for i in at])
+        want2 = orc.OracleIndex(built.bits, built.n_bits).search_reads(l2, r2, k, p)
+        assert np.array_equal(pos.cpu().numpy().view(np.uint64), want2)
