@@ -323,14 +323,17 @@ __global__ void walk_check_kernel(u32 n, u32 k, const u64 *__restrict__ keys, co
     if (!ok) atomicAdd(bad, 1ull);
 }
 
-// Letters of the q-mers: the smallest q with 4^q >= 4 n, so that at most a
-// quarter of the q-mers of random letters are present, as long as the bitmap
-// (4^q bits) is no larger than 32 MiB (q = 14), where it stays in L2 next to
-// the lines; larger indexes keep q = 14 up to 4^14 columns, then take the
-// smallest q with 4^q > n.
+// Letters of the q-mers: the smallest q with 4^q >= 16 n, so that at most one in
+// 16 q-mers of random letters is present, as long as the bitmap (4^q bits) is no
+// larger than 32 MiB (q = 14), where it still hits L2; larger indexes keep q = 14
+// up to 4^14 columns, then take the smallest q with 4^q >= n.  Measured at 1M
+// columns with the limit at 2 n or 4 n (q = 11), 8 n or 16 n (q = 12) and 64 n
+// (q = 13): 100M single k-mers 949 / 844 / 802 us, uneven reads 2092 / 1955 /
+// 1951, 10,000 reads 95 / 87 / 89; at 4M columns (13 for 16 n, 14 for 64 n) 284 /
+// 300.
 u32 walk_q(u64 n, u32 k) {
     u32 q = 1;
-    while (q < 14u && (1ull << (2u * q)) < 4ull * n) q++;
+    while (q < 14u && (1ull << (2u * q)) < 16ull * n) q++;
     while (q < 16u && (1ull << (2u * q)) < n) q++;
     return q < k ? q : k;
 }
