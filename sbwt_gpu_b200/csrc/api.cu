@@ -575,10 +575,11 @@ int enqueue_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_l
                  u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s, bool prof);
 
 int search_rows_device(sbwt_index *ix, Workspace &w, const uint8_t *d_letters, u64 n_letters, const u64 *d_rows,
-                       u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s) {
+                       u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s, bool found_only) {
     if (n_rows == 0 || n_kmers == 0) return 0;
     const u64 n_words = (n_letters + 32 + 31) / 32;
     SearchArgs a = base_args(ix, true, n_kmers);
+    a.found_only = found_only;
     if (!d_answers && !a.runs) {  // membership only: the per-k-mer kernels derive it from answers
         SBWT_TRY(grow(w.answers, w.answers_cap, n_kmers));
         d_answers = w.answers;
@@ -639,9 +640,10 @@ int prepare_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_l
     SBWT_TRY(grow(w.scan, w.scan_cap, scan_scratch_words(n_rows)));
     SBWT_TRY(grow(w.chunk_row, w.chunk_cap, (n_kmers + a.chunk - 1) / a.chunk));
     SBWT_TRY(grow(w.counter, w.counter_cap, 1));
-    SBWT_TRY(launch_pack(d_letters, n_letters, w.words, s));
-    SBWT_TRY(launch_kstart(d_rows, n_rows, ix->k, w.kstart, w.scan, s));
-    SBWT_TRY(launch_chunk_rows(w.kstart, n_rows, n_kmers, a.chunk, w.chunk_row, s));
+    bool cleared = false;
+    SBWT_TRY(launch_prep(d_letters, n_letters, w.words, d_rows, n_rows, ix->k, w.kstart, w.scan, n_kmers, a.chunk,
+                         w.chunk_row, w.counter, &cleared, s));
+    a.cleared = cleared;
     a.words = w.words;
     a.positions = nullptr;
     a.row_starts = d_rows;
@@ -658,12 +660,19 @@ int prepare_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_l
 int enqueue_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_letters, u64 n_letters, const u64 *d_rows,
                  u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s, bool prof) {
     const u64 n_words = (n_letters + 32 + 31) / 32;
-    if (prof) SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[0], s));
-    SBWT_TRY(launch_pack(d_letters, n_letters, w.words, s));
-    if (prof) SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[1], s));
-    SBWT_TRY(launch_kstart(d_rows, n_rows, ix->k, w.kstart, w.scan, s));
-    SBWT_TRY(launch_chunk_rows(w.kstart, n_rows, n_kmers, a.chunk, w.chunk_row, s));
-    if (prof) SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[2], s));
+    if (prof) {  // the phases one by one
+        SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[0], s));
+        SBWT_TRY(launch_pack(d_letters, n_letters, w.words, s));
+        SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[1], s));
+        SBWT_TRY(launch_kstart(d_rows, n_rows, ix->k, w.kstart, w.scan, s));
+        SBWT_TRY(launch_chunk_rows(w.kstart, n_rows, n_kmers, a.chunk, w.chunk_row, s));
+        SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[2], s));
+    } else {
+        bool cleared = false;
+        SBWT_TRY(launch_prep(d_letters, n_letters, w.words, d_rows, n_rows, ix->k, w.kstart, w.scan, n_kmers, a.chunk,
+                             w.chunk_row, w.counter, &cleared, s));
+        a.cleared = cleared;
+    }
     a.words = w.words;
     a.positions = nullptr;
     a.row_starts = d_rows;
@@ -682,7 +691,7 @@ int enqueue_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_l
     if (member_pass) SBWT_TRY(launch_member_bits(d_answers, n_kmers, d_member, s));
     if (prof) {
         SBWT_CHECK_CUDA(cudaEventRecord(ix->prof_ev[4], s));
-        ix->prof_launches = 1 + 3 + 1 + 1 + (member_pass ? 1 : 0);
+        ix->prof_launches = 1 + 3 + 1 + 1 + (walk_fills(a) ? 1 : 0) + (member_pass ? 1 : 0);
         ix->prof_blocks = blocks;
         ix->prof_member = member_pass;
     }

@@ -43,7 +43,9 @@ struct SearchArgs {
     u64 *answers;
     u64 n_kmers;
     unsigned long long *counter;  // work-stealing cursor (zeroed before launch)
+    u32 cleared;                  // counter is zero already (launch_prep)
     u32 chunk;                    // k-mers per grab; with `runs`, k-mers per window of chunk_row
+    u32 found_only;               // with `walk`: answers of absent k-mers need not be written
     u32 piece;                    // with `walk`: k-mers per run at most
     u32 runs;                     // read mode: walk runs right to left with the absent-run skip
     u32 stream;                   // with `runs`: backward steps from a found k-mer (needs sv)
@@ -212,6 +214,9 @@ int launch_kstart(const uint64_t *d_row_starts, uint64_t n_rows, uint32_t k, uin
 uint64_t scan_scratch_words(uint64_t n_items);
 int launch_chunk_rows(const uint64_t *d_kstart, uint64_t n_rows, uint64_t n_kmers, uint32_t chunk,
                       uint32_t *d_chunk_row, cudaStream_t s);
+int launch_prep(const uint8_t *d_letters, uint64_t n_letters, uint64_t *d_words, const uint64_t *d_row_starts,
+                uint64_t n_rows, uint32_t k, uint64_t *d_kstart, uint64_t *d_scan, uint64_t n_kmers, uint32_t chunk,
+                uint32_t *d_chunk_row, unsigned long long *d_counter, bool *cleared, cudaStream_t s);
 int launch_member_bits(const uint64_t *d_answers, uint64_t n, uint32_t *d_bits, cudaStream_t s);
 // The k-mers j0 .. j0+count-1 of the batch of reads described by a (words,
 // row_starts, kstart, chunk_row, chunk, max_pos) as a list of 64-bit windows.
@@ -239,8 +244,10 @@ SearchArgs base_args(const sbwt_index *ix, bool rows, u64 n_kmers, bool filtered
 // chunk table on s; fills the batch fields of a (a.chunk set by base_args).
 int prepare_rows(sbwt_index *ix, Workspace &w, SearchArgs &a, const uint8_t *d_letters, uint64_t n_letters,
                  const uint64_t *d_rows, uint64_t n_rows, uint64_t n_kmers, cudaStream_t s);
+// found_only: the answers of absent k-mers need not be written (the caller reads those that the bitmap names).
 int search_rows_device(sbwt_index *ix, Workspace &w, const uint8_t *d_letters, u64 n_letters, const u64 *d_rows,
-                       u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s);
+                       u64 n_rows, u64 *d_answers, uint32_t *d_member, u64 n_kmers, cudaStream_t s,
+                       bool found_only = false);
 template <class T> int grow(T *&p, size_t &cap, size_t need);
 template <class T> int grow_host(T *&p, size_t &cap, size_t need);
 
@@ -271,6 +278,7 @@ bool run32_ok(const SearchArgs &a);
 // walk.cu
 u32 walk_chunk(const sbwt_index *ix, u64 n_kmers);
 int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *launched_blocks);
+bool walk_fills(const SearchArgs &a);  // the walk's launch writes the absent answers ahead (a kernel of its own)
 int launch_list(const sbwt_index *ix, SearchArgs &a, cudaStream_t s);
 
 }  // namespace sbwt

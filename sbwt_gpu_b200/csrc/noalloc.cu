@@ -96,12 +96,13 @@ extern "C" int sbwt_search_reads_noalloc(sbwt_index *ix, const uint8_t *d_letter
     u64 *const words = (u64 *)(base + off_words);
     if (scratch_answers) d_answers = (u64 *)(base + off_answers);
 
-    SBWT_TRY(launch_pack(d_letters, n_letters, words, s));
     a.counter = (unsigned long long *)base;  // launch_search clears it on the stream before the kernel
     a.kstart = (u64 *)(base + off_kstart);
     a.chunk_row = (u32 *)(base + off_chunks);
-    SBWT_TRY(launch_kstart(d_row_starts, n_rows, ix->k, (u64 *)(base + off_kstart), (u64 *)(base + off_scan), s));
-    SBWT_TRY(launch_chunk_rows(a.kstart, n_rows, n_kmers, a.chunk, (u32 *)(base + off_chunks), s));
+    bool cleared = false;
+    SBWT_TRY(launch_prep(d_letters, n_letters, words, d_row_starts, n_rows, ix->k, (u64 *)(base + off_kstart),
+                         (u64 *)(base + off_scan), n_kmers, a.chunk, (u32 *)(base + off_chunks), a.counter, &cleared, s));
+    a.cleared = cleared;
     a.member = a.runs ? d_member_bits : nullptr;
     a.words = words;
     a.row_starts = d_row_starts;

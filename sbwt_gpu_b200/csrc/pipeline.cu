@@ -598,7 +598,7 @@ int pipeline_chunks(sbwt_index *ix, const uint8_t *letters, uint64_t n_letters, 
         stage[slot] = 1;
         if (answers && !dense_chunk(b)) {
             // answers and bitmap in one search, then the found node ids gathered per group
-            SBWT_TRY(search_rows_device(ix, w, w.letters, nl, w.rows, nr, w.answers, w.member, c.nk, s));
+            SBWT_TRY(search_rows_device(ix, w, w.letters, nl, w.rows, nr, w.answers, w.member, c.nk, s, true));
             if (c.nk) {
                 const u64 nw = (c.nk + 31) / 32, ng = (nw + kGroupWords - 1) / kGroupWords;
                 u64 *goff = w.goff;

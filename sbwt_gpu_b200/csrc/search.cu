@@ -720,7 +720,7 @@ int launch_one(const R &rk, SearchArgs &a, const sbwt_index *ix, cudaStream_t s,
     if (per_sm < 1) per_sm = 1;
     const u32 blocks = (u32)per_sm * (u32)ix->num_sms;
     if (blocks_out) *blocks_out = blocks;
-    SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
+    if (!a.cleared) SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
     SBWT_TRY(launch_kernel(kern, blocks, tpb, s, ix, rk, a));
     return 0;
 }
@@ -763,7 +763,7 @@ int launch_queue(const R &rk, SearchArgs &a, const sbwt_index *ix, cudaStream_t 
     if (ix->shape.blocks_per_sm && (int)ix->shape.blocks_per_sm < per_sm) per_sm = (int)ix->shape.blocks_per_sm;
     const u32 blocks = (u32)per_sm * (u32)ix->num_sms;
     if (blocks_out) *blocks_out = blocks;
-    SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
+    if (!a.cleared) SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
     SBWT_TRY(launch_kernel(kern, blocks, 128u, s, ix, rk, a));
     return 0;
 }

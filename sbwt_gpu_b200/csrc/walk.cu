@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                             cj = (IX)base;
                             ce = (IX)min((u64)base + a.chunk, (u64)n_eff);
                             crow = a.chunk_row[base / a.chunk];
-                            if (a.answers && a.n_kmers < kFillAhead)
+                            if (a.answers && !a.found_only && a.n_kmers < kFillAhead)
                                 for (u64 t = base + lane; t < ce; t += 32u) a.answers[t] = ~0ull;
                             if (a.member)  // base is a multiple of 32
                                 for (u64 t = base / 32u + lane; t < ((u64)ce + 31u) / 32u; t += 32u) a.member[t] = 0u;
@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                             crow += __shfl_sync(kFull, own, total - 1u);
                         } else {
                             crow += 32u;
+                            if (crow >= (IX)n_rows) cj = ce;  // a row table that does not add up: never a wait for its rows
                         }
                     }
                     __syncwarp();
@@ -545,6 +546,8 @@ u32 walk_chunk(const sbwt_index *ix, u64 n_kmers) {
     return c;
 }
 
+bool walk_fills(const SearchArgs &a) { return a.walk && a.answers && !a.found_only && a.n_kmers >= kFillAhead; }
+
 int launch_list(const sbwt_index *ix, SearchArgs &a, cudaStream_t s) {
     int per_sm = 0;
     SBWT_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, list_kernel, kWarps * 32, 0));
@@ -566,8 +569,8 @@ int launch_walk(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *b
     const u64 need = (a.n_kmers + (u64)a.chunk * kWarps - 1) / ((u64)a.chunk * kWarps);
     const u32 blocks = (u32)std::min<u64>((u64)per_sm * (u64)ix->num_sms, need);
     if (blocks_out) *blocks_out = blocks;
-    SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
-    if (a.answers && a.n_kmers >= kFillAhead) {
+    if (!a.cleared) SBWT_CHECK_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s));
+    if (walk_fills(a)) {
         const u64 per = 4ull * kFillThreads * kFillStores;
         fill_kernel<<<(unsigned)((a.n_kmers + per - 1) / per), kFillThreads, 0, s>>>(a.answers, a.n_kmers, a.runs_dev, a.kstart, a.n_rows);
         SBWT_CHECK_CUDA(cudaGetLastError());

@@ -80,6 +80,32 @@ def test_walk_batch_sizes(cuda, reads):
         assert np.array_equal(_search(ix, letters, rows, want.size, 1), want)
 
 
+@pytest.mark.parametrize("rows", [11_263, 11_264])  # the most rows of the one-launch row table, and one more
+@pytest.mark.parametrize("offset", [0, 16, 1])  # alignment of the letters
+def test_row_tables(cuda, rows, offset):
+    import torch
+    rng = wl.rng_for(rows)
+    k, p = 21, 8
+    genome = wl.random_bases(rng, 30_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    lens = rng.integers(0, 90, size=rows)
+    lens[rng.integers(0, rows, size=rows // 3)] = 0
+    starts = np.zeros(rows + 1, dtype=np.uint64)
+    starts[1:] = np.cumsum(lens)
+    letters = np.resize(genome, int(starts[-1])).copy()
+    wl.substitute(rng, letters, 0.02)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, starts, k, p)
+    buf = torch.zeros(letters.size + offset, dtype=torch.uint8, device="cuda")
+    buf[offset:] = torch.from_numpy(letters).cuda()
+    d_rows = torch.from_numpy(starts.view(np.int64)).cuda()
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        ans = torch.full((want.size + 1,), -7, dtype=torch.int64, device="cuda")
+        ix.search_reads(buf[offset:], d_rows, ans, want.size)
+        torch.cuda.synchronize()
+        got = ans.cpu().numpy().view(np.uint64)
+        assert np.array_equal(got[:-1], want) and got[-1] == np.uint64(2**64 - 7)
+
+
 @pytest.mark.parametrize("dk", [-2, 1])
 def test_another_k_than_the_index(cuda, dk):
     """Searched with a k that is not the one of its labels, an index takes the walk without the labels; the
