@@ -73,46 +73,59 @@ struct Train {
     float *loss_sum = nullptr, *loss_hist = nullptr;
     unsigned long long *step = nullptr;
     int *err = nullptr;
-    std::vector<void *> owned;
+    uint8_t *arena = nullptr;  // all of the above: one allocation, not one each (25 took 10-25 ms a call)
 
-    template <class T>
-    int alloc(T *&p, size_t count) {
-        SBWT_CHECK_CUDA(cudaMalloc((void **)&p, std::max<size_t>(count, 1) * sizeof(T)));
-        owned.push_back((void *)p);
-        return 0;
-    }
-    int setup(uint32_t batch, uint32_t kk, uint32_t hist) {
+    // Places the buffers one after the other in the arena, which is allocated in between the two passes.
+    struct Layout {
+        uint8_t *base;
+        size_t at;
+        template <class T> void put(T *&p, size_t count) {
+            p = reinterpret_cast<T *>(base + at);
+            at += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+        }
+    };
+    // own_batch: room for the batch's k-mers and labels as well.
+    int setup(uint32_t batch, uint32_t kk, uint32_t hist, bool own_batch = false) {
         B = batch;
         k = kk;
         const uint32_t P = off.count;
-        SBWT_TRY(alloc(theta, P));
-        SBWT_TRY(alloc(grad, P));
-        SBWT_TRY(alloc(m, P));
-        SBWT_TRY(alloc(v, P));
-        SBWT_TRY(alloc(W1b, 256 * 128));
-        SBWT_TRY(alloc(W2b, 256 * 256));
-        SBWT_TRY(alloc(W2bT, 256 * 256));
-        SBWT_TRY(alloc(X, (size_t)B * kIn));
-        SBWT_TRY(alloc(XT, (size_t)B * kIn));
-        SBWT_TRY(alloc(H1, (size_t)B * kHid));
-        SBWT_TRY(alloc(H1T, (size_t)B * kHid));
-        SBWT_TRY(alloc(dZ2, (size_t)B * kHid));
-        SBWT_TRY(alloc(dZ2T, (size_t)B * kHid));
-        SBWT_TRY(alloc(dZ1, (size_t)B * kHid));
-        SBWT_TRY(alloc(dZ1T, (size_t)B * kHid));
-        SBWT_TRY(alloc(Y, B));
-        SBWT_TRY(alloc(Z1, (size_t)B * kHid));
-        SBWT_TRY(alloc(Z2, (size_t)B * kHid));
-        SBWT_TRY(alloc(dH1, (size_t)B * kHid));
-        SBWT_TRY(alloc(loss_sum, 1));
-        SBWT_TRY(alloc(loss_hist, hist + 2));
-        SBWT_TRY(alloc(step, 1));
-        SBWT_TRY(alloc(err, 1));
-        SBWT_CHECK_CUDA(cudaMemset(m, 0, P * sizeof(float)));
-        SBWT_CHECK_CUDA(cudaMemset(v, 0, P * sizeof(float)));
-        SBWT_CHECK_CUDA(cudaMemset(step, 0, sizeof(*step)));
-        SBWT_CHECK_CUDA(cudaMemset(err, 0, sizeof(*err)));
-        SBWT_CHECK_CUDA(cudaMemset(loss_hist, 0, (hist + 2) * sizeof(float)));
+        uint64_t *km = nullptr;
+        uint8_t *lb = nullptr;
+        size_t zeroed = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            Layout l{arena, 0};
+            l.put(m, P);
+            l.put(v, P);
+            l.put(loss_hist, hist + 2);
+            l.put(step, 1);
+            l.put(err, 1);
+            zeroed = l.at;
+            l.put(theta, P);
+            l.put(grad, P);
+            l.put(W1b, 256 * 128);
+            l.put(W2b, 256 * 256);
+            l.put(W2bT, 256 * 256);
+            l.put(X, (size_t)B * kIn);
+            l.put(XT, (size_t)B * kIn);
+            l.put(H1, (size_t)B * kHid);
+            l.put(H1T, (size_t)B * kHid);
+            l.put(dZ2, (size_t)B * kHid);
+            l.put(dZ2T, (size_t)B * kHid);
+            l.put(dZ1, (size_t)B * kHid);
+            l.put(dZ1T, (size_t)B * kHid);
+            l.put(Y, B);
+            l.put(Z1, (size_t)B * kHid);
+            l.put(Z2, (size_t)B * kHid);
+            l.put(dH1, (size_t)B * kHid);
+            l.put(loss_sum, 1);
+            if (own_batch) {
+                l.put(km, B);
+                l.put(lb, B);
+            }
+            if (pass == 0) SBWT_CHECK_CUDA(cudaMalloc((void **)&arena, l.at));
+        }
+        if (own_batch) kmers = km, labels = lb, n_train = B;
+        SBWT_CHECK_CUDA(cudaMemset(arena, 0, zeroed));
         return 0;
     }
     // the BF16 operand copies of W1 and W2 from theta
@@ -122,9 +135,7 @@ struct Train {
         SBWT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }
-    ~Train() {
-        for (void *p : owned) cudaFree(p);
-    }
+    ~Train() { cudaFree(arena); }
 };
 
 // One training step (forward, loss, backward, and optionally Adam).
@@ -584,14 +595,9 @@ extern "C" int sbwt_mlp_gradients(uint32_t k, const float *theta, const uint64_t
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return set_error("no CUDA device is available");
     Train t;
-    SBWT_TRY(t.setup(n, k, 1));
-    uint64_t *d_k = nullptr;
-    uint8_t *d_l = nullptr;
-    SBWT_TRY(t.alloc(d_k, n));
-    SBWT_TRY(t.alloc(d_l, n));
-    t.kmers = d_k;
-    t.labels = d_l;
-    t.n_train = n;
+    SBWT_TRY(t.setup(n, k, 1, true));
+    uint64_t *d_k = const_cast<uint64_t *>(t.kmers);
+    uint8_t *d_l = const_cast<uint8_t *>(t.labels);
     SBWT_CHECK_CUDA(cudaMemcpy(d_k, kmers, (size_t)n * 8, cudaMemcpyHostToDevice));
     SBWT_CHECK_CUDA(cudaMemcpy(d_l, labels, n, cudaMemcpyHostToDevice));
     SBWT_CHECK_CUDA(cudaMemcpy(t.theta, theta, t.off.count * sizeof(float), cudaMemcpyHostToDevice));
