@@ -61,12 +61,12 @@ template <int ALIGN, u32 THREADS>
 __device__ __forceinline__ void pack_block(const uint8_t *__restrict__ letters, u64 n_letters, u64 *__restrict__ words,
                                            u64 n_words, u64 block) {
     const u64 w0 = block * (THREADS * kPackWords) + threadIdx.x;
-    const u64 whole = ALIGN == 1 ? 0 : n_letters / 32u;
+    const u64 whole = n_letters / 32u;  // words inside the letters
     uint4 v[kPackWords][2];
 #pragma unroll
     for (u32 i = 0; i < kPackWords; i++) {
         const u64 w = w0 + i * THREADS;
-        if (w >= whole) continue;
+        if (ALIGN == 1 || w >= whole) continue;
         const uint4 *p = reinterpret_cast<const uint4 *>(letters + w * 32u);
         if constexpr (ALIGN == 32) {
             asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -81,7 +81,7 @@ __device__ __forceinline__ void pack_block(const uint8_t *__restrict__ letters, 
 #pragma unroll
     for (u32 i = 0; i < kPackWords; i++) {
         const u64 w = w0 + i * THREADS;
-        if (w < whole) {
+        if (ALIGN != 1 && w < whole) {
             words[w] = pack32(v[i][0], v[i][1]);
         } else if (w < n_words) {
             u64 x = 0;

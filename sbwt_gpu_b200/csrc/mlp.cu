@@ -19,22 +19,73 @@ namespace sbwt {
 namespace mlp {
 
 using namespace tc;
+using u16 = uint16_t;
 
 // ------------------------------------------------------------------ GEMM
 
-// D[M x N] (+)= A[M x K] * B[N x K]^T for the K range of blockIdx.z; A and B
-// row-major BF16, M a multiple of 128, N of BN, K of 64.  128 threads.
-template <u32 BN>
-__global__ void __launch_bounds__(128) gemm_tn_kernel(const bf16 *__restrict__ A, const bf16 *__restrict__ B,
-                                                      float *__restrict__ D, u32 N, u32 K, u32 kps, int atomic,
-                                                      int *err) {
+// D[M x N] = A[M x K] * B[N x K]^T for the K range of blockIdx.z; A and B
+// row-major BF16, M a multiple of 128, N of BN, K of 64.  128 threads; thread t
+// ends with row m0 + t of the tile in TMEM, and EPI says what becomes of it
+// (TrainEpi).  Training is bound by the number of passes over its 2-8 MB
+// matrices, so every pass that works on one row or writes a transposed copy is
+// done here, from TMEM, where a warp's 32 rows make both forms of a store
+// coalesce: with a kernel for each of them (bias and ReLU, head, ReLU gradient,
+// five transposes, FP32 intermediates between them) a step took 18 launches.
+enum { kEpiAdd, kEpiRelu, kEpiHead, kEpiReluGrad };
+
+// Column sums over a warp's 32 rows: lane l returns the sum of column l & 15 of
+// the lanes' 16 values.
+__device__ __forceinline__ float column_sums(float (&v)[16], u32 lane) {
+#pragma unroll
+    for (u32 w = 8; w; w >>= 1) {
+        const bool up = lane & w;
+#pragma unroll
+        for (u32 i = 0; i < 8u; i++) {
+            if (i >= w) break;
+            const float send = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+__device__ __forceinline__ float warp_sum(float x) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// 16 bf16 values of one row, and the same as a column each of the transposed matrix (`rows` rows apart).
+__device__ __forceinline__ void store_row(bf16 *row, const u32 (&h)[8]) {
+    *reinterpret_cast<uint4 *>(row) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(row + 8) = make_uint4(h[4], h[5], h[6], h[7]);
+}
+
+__device__ __forceinline__ void store_columns(bf16 *first, u32 rows, const u32 (&h)[8]) {
+#pragma unroll
+    for (u32 i = 0; i < 16u; i++) {
+        const u16 x = (u16)(h[i / 2] >> (16u * (i & 1u)));
+        *reinterpret_cast<u16 *>(first + (size_t)i * rows) = x;
+    }
+}
+
+__device__ __forceinline__ float bf16_of(const u32 (&h)[8], u32 i) {
+    return __uint_as_float(i & 1u ? h[i / 2] & 0xffff0000u : h[i / 2] << 16);
+}
+
+template <u32 BN, int EPI>
+__global__ void __launch_bounds__(128) gemm_tn_kernel(const bf16 *__restrict__ A, const bf16 *__restrict__ B, u32 M,
+                                                      u32 N, u32 K, u32 kps, const TrainEpi t, int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t bar;
     __shared__ u32 tmem_s;
+    __shared__ float s_sum[2][BN];  // column sums of the tile
     uint8_t *sA = smem;
     uint8_t *sB = smem + 128 * 64 * 2;
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const u32 m0 = blockIdx.x * 128u, n0 = blockIdx.y * BN;
+    if constexpr (EPI == kEpiHead || EPI == kEpiReluGrad)
+        for (u32 i = tid; i < BN; i += 128u) s_sum[0][i] = s_sum[1][i] = 0.0f;
     const u32 kbeg = blockIdx.z * kps, kend = min(K, kbeg + kps);
     constexpr u32 kCols = BN < 32 ? 32 : BN;
     if (warp == 0) tmem_alloc(&tmem_s, kCols);
@@ -46,11 +97,13 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(const bf16 *__restrict__ A
     u32 phase = 0;
     bool ok = true;
     for (u32 kb = kbeg; kb < kend && ok; kb += 64) {
+#pragma unroll
         for (u32 i = tid; i < 128u * 8u; i += 128u) {
             const u32 r = i >> 3, kc = i & 7u;
             const uint4 v = *reinterpret_cast<const uint4 *>(A + (size_t)(m0 + r) * K + kb + kc * 8u);
             *reinterpret_cast<uint4 *>(sA + canon_offset(128, r, kc * 8u)) = v;
         }
+#pragma unroll 8
         for (u32 i = tid; i < BN * 8u; i += 128u) {
             const u32 r = i >> 3, kc = i & 7u;
             const uint4 v = *reinterpret_cast<const uint4 *>(B + (size_t)(n0 + r) * K + kb + kc * 8u);
@@ -74,21 +127,92 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(const bf16 *__restrict__ A
         ok = __syncthreads_and(got);
     }
     if (ok && kend > kbeg) {
-        const u32 row = m0 + warp * 32u + lane;
-        for (u32 c = 0; c < BN; c += 16) {
-            u32 v[16];
-            tmem_ld16(tmem + ((warp * 32u) << 16) + c, v);
-            tmem_wait_ld();
-            float *dst = D + (size_t)row * N + n0 + c;
-            if (atomic) {
+        const u32 row = m0 + warp * 32u + lane, acc = tmem + ((warp * 32u) << 16);
+        float dz = 0.0f;
+        if constexpr (EPI == kEpiHead) {
+            // logit of the row: h2 = bf16(ReLU(z2 + b2)), h2 . w3 + b3; BCE with logits: softplus(z) - y z,
+            // d/dz = sigmoid(z) - y
+            float sum = 0.0f;
+            for (u32 c = 0; c < BN; c += 16) {
+                u32 v[16];
+                tmem_ld16(acc + c, v);
+                tmem_wait_ld();
+                tmem_tie(v);
 #pragma unroll
-                for (int j = 0; j < 16; j++) atomicAdd(dst + j, __uint_as_float(v[j]));
-            } else {
+                for (int j = 0; j < 16; j++)
+                    sum = fmaf(bf16_round(fmaxf(__uint_as_float(v[j]) + t.bias[c + j], 0.0f)), t.w3[c + j], sum);
+            }
+            const float z = sum + *t.b3, y = t.labels[row];
+            const float sp = z > 0 ? z + log1pf(expf(-z)) : log1pf(expf(z));
+            dz = (1.0f / (1.0f + expf(-z)) - y) / (float)M;
+            const float loss = warp_sum((sp - y * z) / (float)M), db3 = warp_sum(dz);
+            if (lane == 0) {
+                atomicAdd(t.loss, loss);
+                atomicAdd(t.g_b3, db3);
+            }
+        }
+        for (u32 c = 0; c < BN; c += 16) {
+            u32 v[16], h[8];
+            tmem_ld16(acc + c, v);
+            tmem_wait_ld();
+            tmem_tie(v);
+            if constexpr (EPI == kEpiAdd) {
+                float *dst = t.add + (size_t)row * N + n0 + c;
 #pragma unroll
                 for (int j = 0; j < 16; j += 4)
-                    *reinterpret_cast<float4 *>(dst + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                       __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                    atomicAdd(reinterpret_cast<float4 *>(dst + j),
+                              make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
+                                          __uint_as_float(v[j + 3])));
+            } else if constexpr (EPI == kEpiRelu) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 2)
+                    h[j / 2] = pack_bf16x2(fmaxf(__uint_as_float(v[j]) + t.bias[n0 + c + j], 0.0f),
+                                           fmaxf(__uint_as_float(v[j + 1]) + t.bias[n0 + c + j + 1], 0.0f));
+                store_row(t.out + (size_t)row * N + n0 + c, h);
+                store_columns(t.out_t + (size_t)(n0 + c) * M + row, M, h);
+            } else if constexpr (EPI == kEpiHead) {
+                // dz2 = dlogit * w3 * [h2 > 0]; gradients of w3 and b2: sums over the rows
+                float dw[16], db[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float x = bf16_round(fmaxf(__uint_as_float(v[j]) + t.bias[c + j], 0.0f));
+                    dw[j] = dz * x;
+                    db[j] = x > 0.0f ? dz * t.w3[c + j] : 0.0f;
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) h[j / 2] = pack_bf16x2(db[j], db[j + 1]);
+                store_row(t.out + (size_t)row * N + c, h);
+                store_columns(t.out_t + (size_t)c * M + row, M, h);
+#pragma unroll
+                for (int j = 0; j < 16; j++) db[j] = bf16_of(h, j);
+                const float sw = column_sums(dw, lane), sb = column_sums(db, lane);
+                if (lane < 16) {
+                    atomicAdd(&s_sum[0][c + lane], sw);
+                    atomicAdd(&s_sum[1][c + lane], sb);
+                }
+            } else {
+                // dz1 = dh1 * [h1 > 0], only its transpose is used; gradient of b1: sums over the rows
+                const uint4 *hp = reinterpret_cast<const uint4 *>(t.h + (size_t)row * N + n0 + c);
+                const uint4 h0 = hp[0], h1 = hp[1];
+                const u32 m[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                float g[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) g[j] = bf16_of(m, j) > 0.0f ? __uint_as_float(v[j]) : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) h[j / 2] = pack_bf16x2(g[j], g[j + 1]);
+                store_columns(t.out_t + (size_t)(n0 + c) * M + row, M, h);
+#pragma unroll
+                for (int j = 0; j < 16; j++) g[j] = bf16_of(h, j);
+                const float sb = column_sums(g, lane);
+                if (lane < 16) atomicAdd(&s_sum[1][c + lane], sb);
             }
+        }
+    }
+    if constexpr (EPI == kEpiHead || EPI == kEpiReluGrad) {
+        __syncthreads();
+        for (u32 i = tid; i < BN; i += 128u) {
+            if constexpr (EPI == kEpiHead) atomicAdd(t.g_w3 + i, s_sum[0][i]);
+            atomicAdd(t.g_bias + n0 + i, s_sum[1][i]);
         }
     }
     if (!ok && tid == 0) mbar_wait(&bar, phase ^ 1u, err, kErrGemmWait);  // let an MMA still in flight land
@@ -325,126 +449,44 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 
 // ------------------------------------------------------- training helpers
 
-// X[b] = one-hot of k-mer (batch_start + b), Y[b] = its label.
+// Rows of 8 inputs of X[b] = one-hot of k-mer (batch_start + b) (16 a row), rows
+// of 8 k-mers of its transpose XT, and Y[b] = the label; batch a multiple of 8.
 __global__ void onehot_batch_kernel(const u64 *__restrict__ kmers, const uint8_t *__restrict__ labels, u64 n_train,
                                     const unsigned long long *step, u32 batch, u32 k, bf16 *__restrict__ X,
-                                    float *__restrict__ Y) {
-    const u32 b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch) return;
+                                    bf16 *__restrict__ XT, float *__restrict__ Y) {
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, half = batch * (kIn / 8);
     const u64 start = ((u64)*step * batch) % (n_train - batch + 1);
-    const u64 kmer = kmers[start + b];
-    Y[b] = (float)labels[start + b];
-    uint16_t *row = reinterpret_cast<uint16_t *>(X + (size_t)b * kIn);
-    for (u32 i = 0; i < kIn / 4; i++) {
-        const u32 c = i < k ? letter(kmer, i) : 4u;
+    constexpr u32 one = 0x3F80u;  // bf16 1.0
+    u32 w[4];
+    if (t < half) {
+        const u32 b = t / (kIn / 8), q = t % (kIn / 8);
+        const u64 kmer = kmers[start + b];
+        if (q == 0) Y[b] = (float)labels[start + b];
 #pragma unroll
-        for (u32 j = 0; j < 4; j++) row[4 * i + j] = (c == j) ? 0x3F80 : 0;
-    }
-}
-
-// dst[c][r] = src[r][c] (bf16, 32x32 tiles through shared memory)
-__global__ void transpose_kernel(const bf16 *__restrict__ src, bf16 *__restrict__ dst, u32 R, u32 C) {
-    __shared__ bf16 t[32][33];
-    const u32 c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (u32 i = threadIdx.y; i < 32; i += blockDim.y) {
-        const u32 r = r0 + i, c = c0 + threadIdx.x;
-        if (r < R && c < C) t[i][threadIdx.x] = src[(size_t)r * C + c];
-    }
-    __syncthreads();
-    for (u32 i = threadIdx.y; i < 32; i += blockDim.y) {
-        const u32 c = c0 + i, r = r0 + threadIdx.x;
-        if (r < R && c < C) dst[(size_t)c * R + r] = t[threadIdx.x][i];
-    }
-}
-
-// H = bf16(ReLU(Z + bias)), Z [rows][256] fp32
-__global__ void bias_relu_kernel(const float *__restrict__ Z, const float *__restrict__ bias, bf16 *__restrict__ H,
-                                 u64 count) {
-    const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    H[i] = __float2bfloat16_rn(fmaxf(Z[i] + bias[i % kHid], 0.0f));
-}
-
-// Per row: h2 = bf16(ReLU(z2 + b2)), logit = h2 . w3 + b3, BCE loss;
-// dZ2 = dlogit * w3 * [h2 > 0] (bf16), and the gradients of w3, b3, b2
-// (block-reduced, then atomically added).  One warp per row, 8 rows/block.
-__global__ void __launch_bounds__(256) head_kernel(const float *__restrict__ Z2, const float *__restrict__ theta,
-                                                   const float *__restrict__ Y, u32 batch, bf16 *__restrict__ dZ2,
-                                                   float *__restrict__ grad, float *__restrict__ loss_sum,
-                                                   const MlpOffsets off) {
-    __shared__ float s_dw3[kHid], s_db2[kHid], s_db3;
-    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    for (u32 i = threadIdx.x; i < kHid; i += blockDim.x) { s_dw3[i] = 0.0f; s_db2[i] = 0.0f; }
-    if (threadIdx.x == 0) s_db3 = 0.0f;
-    __syncthreads();
-    const float *b2 = theta + off.b2, *w3 = theta + off.w3;
-    const float b3 = theta[off.b3];
-    const u32 r = blockIdx.x * 8 + warp;
-    if (r < batch) {
-        float h[8], s = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const u32 c = lane * 8 + j;
-            h[j] = bf16_round(fmaxf(Z2[(size_t)r * kHid + c] + b2[c], 0.0f));
-            s = fmaf(h[j], w3[c], s);
+        for (u32 i = 0; i < 4u; i++) {
+            const u32 l = 2u * q + i / 2u, c = l < k ? letter(kmer, l) : 4u, j = 2u * (i & 1u);
+            w[i] = (c == j ? one : 0u) | (c == j + 1u ? one << 16 : 0u);
         }
+        *reinterpret_cast<uint4 *>(X + (size_t)b * kIn + 8u * q) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else if (t < 2u * half) {
+        const u32 u = t - half, i = u / (batch / 8u), b = u % (batch / 8u) * 8u, l = i / 4u, j = i & 3u;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const float z = s + b3, y = Y[r];
-        // BCE with logits: softplus(z) - y z;  d/dz = sigmoid(z) - y
-        const float sp = z > 0 ? z + log1pf(expf(-z)) : log1pf(expf(z));
-        const float sig = 1.0f / (1.0f + expf(-z));
-        const float dz = (sig - y) / (float)batch;
-        if (lane == 0) {
-            atomicAdd(loss_sum, (sp - y * z) / (float)batch);
-            atomicAdd(&s_db3, dz);
+        for (u32 x = 0; x < 4u; x++) {
+            w[x] = 0;
+            if (l < k)
+                w[x] = (letter(kmers[start + b + 2u * x], l) == j ? one : 0u) |
+                       (letter(kmers[start + b + 2u * x + 1u], l) == j ? one << 16 : 0u);
         }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const u32 c = lane * 8 + j;
-            const float g = h[j] > 0.0f ? dz * w3[c] : 0.0f;
-            dZ2[(size_t)r * kHid + c] = __float2bfloat16_rn(g);
-            atomicAdd(&s_dw3[c], dz * h[j]);
-            atomicAdd(&s_db2[c], bf16_round(g));
-        }
+        *reinterpret_cast<uint4 *>(XT + (size_t)i * batch + b) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    __syncthreads();
-    for (u32 i = threadIdx.x; i < kHid; i += blockDim.x) {
-        atomicAdd(grad + off.w3 + i, s_dw3[i]);
-        atomicAdd(grad + off.b2 + i, s_db2[i]);
-    }
-    if (threadIdx.x == 0) atomicAdd(grad + off.b3, s_db3);
-}
-
-// dZ1 = bf16(dH1 * [h1 > 0]); db1 += column sums.  One warp per row.
-__global__ void __launch_bounds__(256) relu_grad_kernel(const float *__restrict__ dH1, const bf16 *__restrict__ H1,
-                                                        u32 batch, bf16 *__restrict__ dZ1, float *__restrict__ grad,
-                                                        const MlpOffsets off) {
-    __shared__ float s_db1[kHid];
-    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    for (u32 i = threadIdx.x; i < kHid; i += blockDim.x) s_db1[i] = 0.0f;
-    __syncthreads();
-    const u32 r = blockIdx.x * 8 + warp;
-    if (r < batch) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const u32 c = lane * 8 + j;
-            const size_t i = (size_t)r * kHid + c;
-            const float g = __bfloat162float(H1[i]) > 0.0f ? dH1[i] : 0.0f;
-            const bf16 gb = __float2bfloat16_rn(g);
-            dZ1[i] = gb;
-            atomicAdd(&s_db1[c], __bfloat162float(gb));
-        }
-    }
-    __syncthreads();
-    for (u32 i = threadIdx.x; i < kHid; i += blockDim.x) atomicAdd(grad + off.b1 + i, s_db1[i]);
 }
 
 // Adam (Kingma & Ba 2015) over the whole parameter vector, then the BF16
-// operand copies of W1 and W2; inputs past 4k of W1 stay zero.
+// operand copies of W1, W2 and W2's transpose; inputs past 4k of W1 stay zero.
 __global__ void adam_kernel(float *__restrict__ theta, const float *__restrict__ grad, float *__restrict__ m,
                             float *__restrict__ v, const unsigned long long *step, u32 count, float lr, u32 k,
-                            bf16 *__restrict__ W1b, bf16 *__restrict__ W2b, const MlpOffsets off) {
+                            bf16 *__restrict__ W1b, bf16 *__restrict__ W2b, bf16 *__restrict__ W2bT,
+                            const MlpOffsets off) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -459,7 +501,10 @@ __global__ void adam_kernel(float *__restrict__ theta, const float *__restrict__
     const float p = theta[i] - lr * mh / (sqrtf(vh) + eps);
     theta[i] = p;
     if (i < off.b1) W1b[i] = __float2bfloat16_rn(p);
-    else if (i >= off.W2 && i < off.b2) W2b[i - off.W2] = __float2bfloat16_rn(p);
+    else if (i >= off.W2 && i < off.b2) {
+        const u32 j = i - off.W2;
+        W2b[j] = W2bT[j % kHid * kHid + j / kHid] = __float2bfloat16_rn(p);
+    }
 }
 
 __global__ void step_kernel(unsigned long long *step, float *loss_hist, const float *loss_sum, u32 hist_every) {
@@ -468,9 +513,14 @@ __global__ void step_kernel(unsigned long long *step, float *loss_hist, const fl
     *step = s + 1;
 }
 
-__global__ void to_bf16_kernel(const float *__restrict__ src, bf16 *__restrict__ dst, u32 count) {
+// dst_t: NULL, or the transpose of src as rows of `cols`.
+__global__ void to_bf16_kernel(const float *__restrict__ src, bf16 *__restrict__ dst, u32 count,
+                               bf16 *__restrict__ dst_t, u32 cols) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) dst[i] = __float2bfloat16_rn(src[i]);
+    if (i >= count) return;
+    const bf16 x = __float2bfloat16_rn(src[i]);
+    dst[i] = x;
+    if (dst_t) dst_t[i % cols * (count / cols) + i / cols] = x;
 }
 
 // ------------------------------------------------- k-mers from the index
@@ -596,32 +646,41 @@ __global__ void accuracy_kernel(const float *__restrict__ logits, const uint8_t 
 
 // ------------------------------------------------------------ launchers
 
-int gemm_tn(const bf16 *A, const bf16 *B, float *D, u32 M, u32 N, u32 K, u32 splits, int *err, cudaStream_t s) {
-    if (M % 128 || K % 64 || (N != 128 && N != 256)) return set_error("gemm_tn: unsupported shape %ux%ux%u", M, N, K);
+namespace {
+
+template <u32 BN, int EPI>
+int launch_gemm(const bf16 *A, const bf16 *B, u32 M, u32 N, u32 K, u32 splits, const TrainEpi &t, int *err,
+                cudaStream_t s) {
+    if (M % 128 || K % 64 || N % BN) return set_error("gemm: unsupported shape %ux%ux%u", M, N, K);
     const u32 ksteps = K / 64;
     splits = std::max(1u, std::min(splits, ksteps));
     const u32 kps = ((ksteps + splits - 1) / splits) * 64;
     splits = (K + kps - 1) / kps;
-    const dim3 grid(M / 128, 1, splits);
-    const int atomic = splits > 1;
-    static bool attr_set = false;  // 48 KiB of dynamic shared memory needs the opt-in
-    if (!attr_set) {
-        SBWT_CHECK_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             128 * 64 * 2 + 256 * 64 * 2));
-        SBWT_CHECK_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             128 * 64 * 2 + 128 * 64 * 2));
-        attr_set = true;
-    }
-    if (atomic) SBWT_CHECK_CUDA(cudaMemsetAsync(D, 0, (size_t)M * N * sizeof(float), s));
-    if (N == 256) {
-        const u32 smem = 128 * 64 * 2 + 256 * 64 * 2;
-        gemm_tn_kernel<256><<<grid, 128, smem, s>>>(A, B, D, N, K, kps, atomic, err);
-    } else {
-        const u32 smem = 128 * 64 * 2 + 128 * 64 * 2;
-        gemm_tn_kernel<128><<<grid, 128, smem, s>>>(A, B, D, N, K, kps, atomic, err);
-    }
+    constexpr u32 smem = (128 + BN) * 64 * 2;
+    if (smem > 32768)  // with the static part beyond 48 KiB: the opt-in, a per-device attribute
+        SBWT_CHECK_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    gemm_tn_kernel<BN, EPI><<<dim3(M / 128, N / BN, splits), 128, smem, s>>>(A, B, M, N, K, kps, t, err);
     SBWT_CHECK_CUDA(cudaGetLastError());
     return 0;
+}
+
+}  // namespace
+
+// The products of a training step (prefilter.cu enqueue_step).  Tiles of 128
+// columns where the rows of a result need not be whole: twice the blocks of 256.
+int gemm_relu(const bf16 *A, const bf16 *B, u32 M, u32 K, const TrainEpi &t, int *err, cudaStream_t s) {
+    return launch_gemm<128, kEpiRelu>(A, B, M, kHid, K, 1, t, err, s);
+}
+int gemm_head(const bf16 *A, const bf16 *B, u32 M, const TrainEpi &t, int *err, cudaStream_t s) {
+    return launch_gemm<256, kEpiHead>(A, B, M, kHid, kHid, 1, t, err, s);
+}
+int gemm_relu_grad(const bf16 *A, const bf16 *B, u32 M, const TrainEpi &t, int *err, cudaStream_t s) {
+    return launch_gemm<128, kEpiReluGrad>(A, B, M, kHid, kHid, 1, t, err, s);
+}
+int gemm_add(const bf16 *A, const bf16 *B, u32 N, u32 K, u32 splits, float *D, int *err, cudaStream_t s) {
+    TrainEpi t{};
+    t.add = D;
+    return launch_gemm<128, kEpiAdd>(A, B, kHid, N, K, splits, t, err, s);
 }
 
 int infer(const u64 *kmers, u64 n, u32 k, const bf16 *W1b, const bf16 *W2b, const InferBias &bias,
@@ -639,12 +698,6 @@ int infer(const u64 *kmers, u64 n, u32 k, const bf16 *W1b, const bf16 *W2b, cons
     const u64 tiles = (n + kTileM - 1) / kTileM;
     const u32 grid = (u32)std::min<u64>(tiles, (u64)num_sms);
     mlp_infer_kernel<<<grid, kInferThreads, kInferSmem, s>>>(kmers, n, k, W1b, W2b, bias, out, err);
-    SBWT_CHECK_CUDA(cudaGetLastError());
-    return 0;
-}
-
-int transpose(const bf16 *src, bf16 *dst, u32 R, u32 C, cudaStream_t s) {
-    transpose_kernel<<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(src, dst, R, C);
     SBWT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -27,17 +27,12 @@ struct C5 {
 // Kernels of mlp.cu launched from prefilter.cu (see mlp.cu for each).
 __global__ void onehot_batch_kernel(const uint64_t *kmers, const uint8_t *labels, uint64_t n_train,
                                     const unsigned long long *step, uint32_t batch, uint32_t k, __nv_bfloat16 *X,
-                                    float *Y);
-__global__ void bias_relu_kernel(const float *Z, const float *bias, __nv_bfloat16 *H, uint64_t count);
-__global__ void head_kernel(const float *Z2, const float *theta, const float *Y, uint32_t batch, __nv_bfloat16 *dZ2,
-                            float *grad, float *loss_sum, const MlpOffsets off);
-__global__ void relu_grad_kernel(const float *dH1, const __nv_bfloat16 *H1, uint32_t batch, __nv_bfloat16 *dZ1,
-                                 float *grad, const MlpOffsets off);
+                                    __nv_bfloat16 *XT, float *Y);
 __global__ void adam_kernel(float *theta, const float *grad, float *m, float *v, const unsigned long long *step,
                             uint32_t count, float lr, uint32_t k, __nv_bfloat16 *W1b, __nv_bfloat16 *W2b,
-                            const MlpOffsets off);
+                            __nv_bfloat16 *W2bT, const MlpOffsets off);
 __global__ void step_kernel(unsigned long long *step, float *loss_hist, const float *loss_sum, uint32_t hist_every);
-__global__ void to_bf16_kernel(const float *src, __nv_bfloat16 *dst, uint32_t count);
+__global__ void to_bf16_kernel(const float *src, __nv_bfloat16 *dst, uint32_t count, __nv_bfloat16 *dst_t, uint32_t cols);
 __global__ void sample_kernel(const ulonglong4 *lines, uint32_t lpc, C5 C5v, uint32_t n_nodes, uint32_t k,
                               uint64_t n_pos, uint64_t n_neg, uint64_t seed, uint64_t count, uint64_t *out);
 __global__ void enumerate_kernel(const ulonglong4 *lines, uint32_t lpc, C5 C5v, uint32_t n_nodes, uint32_t k,
@@ -48,8 +43,26 @@ __global__ void bloom_build_kernel(const uint64_t *kmers, const float *logits, u
 __global__ void accuracy_kernel(const float *logits, const uint8_t *labels, uint64_t n, float tau,
                                 unsigned long long *correct);
 
-int gemm_tn(const __nv_bfloat16 *A, const __nv_bfloat16 *B, float *D, uint32_t M, uint32_t N, uint32_t K,
-            uint32_t splits, int *err, cudaStream_t s);
+// What the rows of a product become (mlp.cu gemm_tn_kernel).
+struct TrainEpi {
+    float *add;                       // += (FP32, atomically: the products are split along K)
+    const float *bias, *w3, *b3;      // of this layer; output weights and bias (head)
+    const float *labels;              // head
+    const __nv_bfloat16 *h;           // ReLU gradient: the activations it masks by
+    __nv_bfloat16 *out, *out_t;       // BF16 result, row-major and transposed
+    float *g_bias, *g_w3, *g_b3, *loss;  // gradients and loss, added to
+};
+// out = bf16(ReLU(A B^T + bias)), M x 256, and its transpose.
+int gemm_relu(const __nv_bfloat16 *A, const __nv_bfloat16 *B, uint32_t M, uint32_t K, const TrainEpi &t, int *err,
+              cudaStream_t s);
+// Layer 2, loss and the gradient back to its pre-activations (out, out_t), with those of w3, b3 and the bias.
+int gemm_head(const __nv_bfloat16 *A, const __nv_bfloat16 *B, uint32_t M, const TrainEpi &t, int *err, cudaStream_t s);
+// out_t = bf16(A B^T * [h > 0])^T, and the gradient of the bias.
+int gemm_relu_grad(const __nv_bfloat16 *A, const __nv_bfloat16 *B, uint32_t M, const TrainEpi &t, int *err,
+                   cudaStream_t s);
+// D += A B^T, 256 x N.
+int gemm_add(const __nv_bfloat16 *A, const __nv_bfloat16 *B, uint32_t N, uint32_t K, uint32_t splits, float *D, int *err,
+             cudaStream_t s);
 // Outputs of an inference pass: the logits (NULL: not written) and/or the
 // sandwich's reject bitmap (bit j%32 of word j/32 = k-mer j rejected by the
 // model at tau and by the backup Bloom filter; NULL: not written).
@@ -84,7 +97,6 @@ inline void bias_from_host(const float *theta, const MlpOffsets &off, InferBias 
 
 int infer(const uint64_t *kmers, uint64_t n, uint32_t k, const __nv_bfloat16 *W1b, const __nv_bfloat16 *W2b,
           const InferBias &bias, const InferOut &out, int *err, int num_sms, cudaStream_t s);
-int transpose(const __nv_bfloat16 *src, __nv_bfloat16 *dst, uint32_t R, uint32_t C, cudaStream_t s);
 
 }  // namespace mlp
 }  // namespace sbwt

@@ -67,9 +67,8 @@ struct Train {
     const uint8_t *labels = nullptr;
     float *theta = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     bf16 *W1b = nullptr, *W2b = nullptr, *W2bT = nullptr;
-    bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1 = nullptr,
-         *dZ1T = nullptr;
-    float *Y = nullptr, *Z1 = nullptr, *Z2 = nullptr, *dH1 = nullptr;
+    bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1T = nullptr;
+    float *Y = nullptr;
     float *loss_sum = nullptr, *loss_hist = nullptr;
     unsigned long long *step = nullptr;
     int *err = nullptr;
@@ -101,7 +100,7 @@ struct Train {
             l.put(err, 1);
             zeroed = l.at;
             l.put(theta, P);
-            l.put(grad, P);
+            l.put(grad, P + 1);  // and the loss: cleared together
             l.put(W1b, 256 * 128);
             l.put(W2b, 256 * 256);
             l.put(W2bT, 256 * 256);
@@ -111,27 +110,23 @@ struct Train {
             l.put(H1T, (size_t)B * kHid);
             l.put(dZ2, (size_t)B * kHid);
             l.put(dZ2T, (size_t)B * kHid);
-            l.put(dZ1, (size_t)B * kHid);
             l.put(dZ1T, (size_t)B * kHid);
             l.put(Y, B);
-            l.put(Z1, (size_t)B * kHid);
-            l.put(Z2, (size_t)B * kHid);
-            l.put(dH1, (size_t)B * kHid);
-            l.put(loss_sum, 1);
             if (own_batch) {
                 l.put(km, B);
                 l.put(lb, B);
             }
             if (pass == 0) SBWT_CHECK_CUDA(cudaMalloc((void **)&arena, l.at));
         }
+        loss_sum = grad + P;
         if (own_batch) kmers = km, labels = lb, n_train = B;
         SBWT_CHECK_CUDA(cudaMemset(arena, 0, zeroed));
         return 0;
     }
-    // the BF16 operand copies of W1 and W2 from theta
+    // the BF16 operand copies of W1, W2 and W2's transpose from theta
     int refresh_bf16(cudaStream_t s) {
-        to_bf16_kernel<<<(256 * 128 + 255) / 256, 256, 0, s>>>(theta + off.W1, W1b, 256 * 128);
-        to_bf16_kernel<<<(256 * 256 + 255) / 256, 256, 0, s>>>(theta + off.W2, W2b, 256 * 256);
+        to_bf16_kernel<<<(256 * 128 + 255) / 256, 256, 0, s>>>(theta + off.W1, W1b, 256 * 128, nullptr, 128);
+        to_bf16_kernel<<<(256 * 256 + 255) / 256, 256, 0, s>>>(theta + off.W2, W2b, 256 * 256, W2bT, 256);
         SBWT_CHECK_CUDA(cudaGetLastError());
         return 0;
     }
@@ -141,27 +136,35 @@ struct Train {
 // One training step (forward, loss, backward, and optionally Adam).
 int enqueue_step(Train &t, cudaStream_t s, bool adam, float lr, uint32_t hist_every) {
     const uint32_t B = t.B;
-    const int splits = std::max<int>(1, (int)(B / 256));
-    SBWT_CHECK_CUDA(cudaMemsetAsync(t.grad, 0, t.off.count * sizeof(float), s));
-    SBWT_CHECK_CUDA(cudaMemsetAsync(t.loss_sum, 0, sizeof(float), s));
-    onehot_batch_kernel<<<(B + 127) / 128, 128, 0, s>>>(t.kmers, t.labels, t.n_train, t.step, B, t.k, t.X, t.Y);
-    SBWT_TRY(gemm_tn(t.X, t.W1b, t.Z1, B, kHid, kIn, 1, t.err, s));  // Z1 = X W1^T
-    bias_relu_kernel<<<(unsigned)(((size_t)B * kHid + 255) / 256), 256, 0, s>>>(t.Z1, t.theta + t.off.b1, t.H1,
-                                                                                (size_t)B * kHid);
-    SBWT_TRY(gemm_tn(t.H1, t.W2b, t.Z2, B, kHid, kHid, 1, t.err, s));  // Z2 = H1 W2^T
-    head_kernel<<<(B + 7) / 8, 256, 0, s>>>(t.Z2, t.theta, t.Y, B, t.dZ2, t.grad, t.loss_sum, t.off);
-    SBWT_TRY(transpose(t.W2b, t.W2bT, kHid, kHid, s));
-    SBWT_TRY(gemm_tn(t.dZ2, t.W2bT, t.dH1, B, kHid, kHid, 1, t.err, s));  // dH1 = dZ2 W2
-    relu_grad_kernel<<<(B + 7) / 8, 256, 0, s>>>(t.dH1, t.H1, B, t.dZ1, t.grad, t.off);
-    SBWT_TRY(transpose(t.dZ2, t.dZ2T, B, kHid, s));
-    SBWT_TRY(transpose(t.H1, t.H1T, B, kHid, s));
-    SBWT_TRY(gemm_tn(t.dZ2T, t.H1T, t.grad + t.off.W2, kHid, kHid, B, splits, t.err, s));  // dW2 = dZ2^T H1
-    SBWT_TRY(transpose(t.dZ1, t.dZ1T, B, kHid, s));
-    SBWT_TRY(transpose(t.X, t.XT, B, kIn, s));
-    SBWT_TRY(gemm_tn(t.dZ1T, t.XT, t.grad + t.off.W1, kHid, kIn, B, splits, t.err, s));  // dW1 = dZ1^T X
+    SBWT_CHECK_CUDA(cudaMemsetAsync(t.grad, 0, (t.off.count + 1) * sizeof(float), s));  // and the loss
+    onehot_batch_kernel<<<(2 * B * (kIn / 8) + 255) / 256, 256, 0, s>>>(t.kmers, t.labels, t.n_train, t.step, B, t.k,
+                                                                        t.X, t.XT, t.Y);
+    TrainEpi e1{}, e2{}, e3{};
+    e1.bias = t.theta + t.off.b1;
+    e1.out = t.H1;
+    e1.out_t = t.H1T;
+    SBWT_TRY(gemm_relu(t.X, t.W1b, B, kIn, e1, t.err, s));  // H1 = ReLU(X W1^T + b1)
+    e2.bias = t.theta + t.off.b2;
+    e2.w3 = t.theta + t.off.w3;
+    e2.b3 = t.theta + t.off.b3;
+    e2.labels = t.Y;
+    e2.out = t.dZ2;
+    e2.out_t = t.dZ2T;
+    e2.g_bias = t.grad + t.off.b2;
+    e2.g_w3 = t.grad + t.off.w3;
+    e2.g_b3 = t.grad + t.off.b3;
+    e2.loss = t.loss_sum;
+    SBWT_TRY(gemm_head(t.H1, t.W2b, B, e2, t.err, s));  // Z2 = H1 W2^T, loss, dZ2
+    e3.h = t.H1;
+    e3.out_t = t.dZ1T;
+    e3.g_bias = t.grad + t.off.b1;
+    SBWT_TRY(gemm_relu_grad(t.dZ2, t.W2bT, B, e3, t.err, s));  // dZ1 = dZ2 W2 [H1 > 0]
+    // about two blocks an SM, each at least 128 rows of the batch
+    SBWT_TRY(gemm_add(t.dZ2T, t.H1T, kHid, B, std::min(B / 128u, 64u), t.grad + t.off.W2, t.err, s));  // dZ2^T H1
+    SBWT_TRY(gemm_add(t.dZ1T, t.XT, kIn, B, std::min(B / 128u, 128u), t.grad + t.off.W1, t.err, s));   // dZ1^T X
     if (adam) {
         adam_kernel<<<(t.off.count + 255) / 256, 256, 0, s>>>(t.theta, t.grad, t.m, t.v, t.step, t.off.count, lr, t.k,
-                                                             t.W1b, t.W2b, t.off);
+                                                             t.W1b, t.W2b, t.W2bT, t.off);
         step_kernel<<<1, 1, 0, s>>>(t.step, t.loss_hist, t.loss_sum, hist_every);
     }
     SBWT_CHECK_CUDA(cudaGetLastError());
@@ -630,8 +633,8 @@ extern "C" int sbwt_mlp_logits(uint32_t k, const float *theta, const uint64_t *k
         cudaMemset(err, 0, sizeof(int));
         cudaMemcpy(d_th, theta, off.count * 4, cudaMemcpyHostToDevice);
         cudaMemcpy(d_k, kmers, n * 8, cudaMemcpyHostToDevice);
-        to_bf16_kernel<<<(256 * 128 + 255) / 256, 256>>>(d_th + off.W1, w1, 256 * 128);
-        to_bf16_kernel<<<(256 * 256 + 255) / 256, 256>>>(d_th + off.W2, w2, 256 * 256);
+        to_bf16_kernel<<<(256 * 128 + 255) / 256, 256>>>(d_th + off.W1, w1, 256 * 128, nullptr, 128);
+        to_bf16_kernel<<<(256 * 256 + 255) / 256, 256>>>(d_th + off.W2, w2, 256 * 256, nullptr, 256);
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
         InferBias hb;
