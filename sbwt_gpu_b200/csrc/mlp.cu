@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(const bf16 *__restrict__ A
 constexpr u32 kInferThreads = 512;
 constexpr u32 kColGroups = kInferThreads / kTileM;  // 4
 constexpr u32 kGroupCols = kHid / kColGroups;       // 64
-constexpr u32 kInferSmem = kHid * kIn * 2 + kHid * kHid * 2 + kTileM * kIn * 2 + kColGroups * kTileM * 4;
+constexpr u32 kInferBlock = kInferThreads + 32;     // and the warp that issues the MMAs
+constexpr u32 kInferSmem = kHid * kIn * 2 + kHid * kHid * 2 + kTileM * kIn * 2 + (kColGroups - 1) * kTileM * 4;
 
 // One-hot chunks q0..q1-1 of row r: chunk q holds inputs 8q..8q+7 = letters
 // 2q and 2q+1 (4 one-hot inputs each).
@@ -237,61 +238,73 @@ __device__ __forceinline__ void onehot_chunks(uint8_t *tile, u32 R, u32 r, u64 k
         const u32 i0 = 2 * q, i1 = 2 * q + 1;
         const u32 c0 = i0 < k ? letter(kmer, i0) : 4u;
         const u32 c1 = i1 < k ? letter(kmer, i1) : 4u;
-        uint4 w;
-        const u32 one = 0x3F80u;  // bf16 1.0
-        w.x = (c0 == 0 ? one : 0u) | ((c0 == 1 ? one : 0u) << 16);
-        w.y = (c0 == 2 ? one : 0u) | ((c0 == 3 ? one : 0u) << 16);
-        w.z = (c1 == 0 ? one : 0u) | ((c1 == 1 ? one : 0u) << 16);
-        w.w = (c1 == 2 ? one : 0u) | ((c1 == 3 ? one : 0u) << 16);
+        // four bf16 0/1 of a letter: 1.0 shifted to its place (past the 64 bits for none)
+        const u64 w0 = c0 < 4u ? 0x3F80ull << (16u * c0) : 0ull, w1 = c1 < 4u ? 0x3F80ull << (16u * c1) : 0ull;
+        const uint4 w = make_uint4((u32)w0, (u32)(w0 >> 32), (u32)w1, (u32)(w1 >> 32));
         *reinterpret_cast<uint4 *>(tile + canon_offset(R, r, 8 * q)) = w;
     }
 }
 
-// One CTA per SM (226 KiB of shared memory, all 512 TMEM columns), 512
-// threads = 16 warps.  The biases and w3 come by value in the parameter
-// space (InferBias, read as float4 through the constant cache).  Warp w
-// reaches TMEM lanes 32*(w%4)..+31 (rows of the 128-k-mer tile) and handles
-// hidden columns 64*(w/4)..+63 of them in both epilogues, so four warps
-// share each row and the epilogues run on all 16 warps; layer 2's 256 -> 1
-// dot is summed over the four column groups in shared memory.
+// BF16 pair of the ReLUs: the maximum of the rounded pair, one instruction instead of two before the rounding.
+__device__ __forceinline__ u32 relu_bf16x2(float lo, float hi) {
+    const __nv_bfloat162 v = __hmax2(__floats2bfloat162_rn(lo, hi), __nv_bfloat162(0.0f, 0.0f));
+    return *reinterpret_cast<const u32 *>(&v);
+}
+
+// One CTA per SM (226 KiB of shared memory, all 512 TMEM columns): 16 epilogue
+// warps and one that issues the MMAs.  The biases and w3 come by value in the
+// parameter space (InferBias, read as float4 through the constant cache).
+// Epilogue warp w reaches TMEM lanes 32*(w%4)..+31 (rows of the 128-k-mer tile);
+// the four warps of a row share its columns, and layer 2's 256 -> 1 dot is summed
+// over them in shared memory.
 //
-// Pipelined over tiles with the TMEM columns in two halves of 256: tile t
-// accumulates in half h (layer 1, then layer 2 over it) and keeps its
-// layer-1 activations (layer 2's A operand, BF16 pairs) in the first 128
-// columns of the other half.  Once layer 2 of tile t has run, that other
-// half is free, so tile t+1's layer-1 MMA runs there while the threads do
-// tile t's layer-2 epilogue, and tile t+1's one-hot tile is built while
-// tile t's layer-2 MMA runs:
-//   epi1(t) -> MMA2(t) || one-hot(t+1) -> MMA1(t+1) || epi2(t) -> epi1(t+1) ...
-// Two mbarriers (layer 1, layer 2), each with its own phase.
-__device__ __forceinline__ void infer_epi1(u32 tacc, u32 ta2, u32 lane_base, u32 c0, const InferBias &bias) {
-    u32 v[4][16];
+// Both layers go in halves of 128 hidden columns, and the TMEM columns in four
+// regions of 128 that rotate by one per tile: layer 1 fills R0 and R1, its
+// activations (layer 2's A operand, BF16 pairs) go to R2, layer 2 accumulates in
+// R3 and, once the first half of layer 1 has been read, in R0; the next tile's
+// layer 1 takes R1 and R2.  So while the epilogue works on one half of layer 1
+// the tensor cores run the other half or the first half (along K) of layer 2, and
+// the next tile's layer 1 runs under the layer-2 epilogue:
+//   MMA:      L1a L1b | L2(k < 128)      L2(k >= 128) | L1a' L1b' | ...
+//   epilogue:     | e1a     e1b   one-hot'       |  e2         | e1a' ...
+// Each hand-over is an mbarrier (one phase a tile), no block-wide barrier.
+//
+// What bounds it are the epilogues: their ALU instructions and, before, their
+// constant loads.  A prefiltered search of 10M k-mers (all but 0.13 ms of it this
+// kernel) took 2.36 ms with whole layers in two halves of TMEM and block barriers;
+// 2.29 as above; 2.26 with the warp's number as a uniform value, so that biases
+// and w3 are loaded by the uniform path (indexed by a register, these loads kept
+// the address unit and the constant cache half busy; as operands at fixed places,
+// in four copies of the loop, they missed the 2 KB immediate-constant cache: 3.59);
+// 2.03 with layer 2's activations rounded in pairs; 1.94 with the ReLU taken on
+// the rounded pair; 1.87 with the one-hot rows made by shifts.
+template <u32 COLS>
+__device__ __forceinline__ void infer_epi1(u32 src, u32 dst, u32 c0, const InferBias &bias) {
+    u32 v[COLS / 16][16];
 #pragma unroll
-    for (u32 j = 0; j < 4; j++) tmem_ld16(tacc + lane_base + c0 + 16u * j, v[j]);
+    for (u32 j = 0; j < COLS / 16; j++) tmem_ld16(src + 16u * j, v[j]);
     tmem_wait_ld();
 #pragma unroll
-    for (u32 j = 0; j < 4; j++) {
+    for (u32 j = 0; j < COLS / 16; j++) {
         tmem_tie(v[j]);
         u32 packed[8];
 #pragma unroll
         for (int t = 0; t < 16; t += 4) {
             // the same 4 biases for every lane of the warp, from the parameter space
             const float4 bb = *reinterpret_cast<const float4 *>(bias.b1 + c0 + 16u * j + t);
-            packed[t / 2] = pack_bf16x2(fmaxf(__uint_as_float(v[j][t]) + bb.x, 0.0f),
-                                        fmaxf(__uint_as_float(v[j][t + 1]) + bb.y, 0.0f));
-            packed[t / 2 + 1] = pack_bf16x2(fmaxf(__uint_as_float(v[j][t + 2]) + bb.z, 0.0f),
-                                            fmaxf(__uint_as_float(v[j][t + 3]) + bb.w, 0.0f));
+            packed[t / 2] = relu_bf16x2(__uint_as_float(v[j][t]) + bb.x, __uint_as_float(v[j][t + 1]) + bb.y);
+            packed[t / 2 + 1] = relu_bf16x2(__uint_as_float(v[j][t + 2]) + bb.z, __uint_as_float(v[j][t + 3]) + bb.w);
         }
-        tmem_st8(ta2 + lane_base + (c0 + 16u * j) / 2u, packed);
+        tmem_st8(dst + 8u * j, packed);
     }
     tmem_wait_st();
 }
 
 // Partial dot of one row's 64 layer-2 activations (bias, ReLU, BF16) with w3.
-__device__ __forceinline__ float infer_epi2(u32 tacc, u32 lane_base, u32 c0, const InferBias &bias) {
+__device__ __forceinline__ float infer_epi2(u32 src, u32 c0, const InferBias &bias) {
     u32 v[4][16];
 #pragma unroll
-    for (u32 j = 0; j < 4; j++) tmem_ld16(tacc + lane_base + c0 + 16u * j, v[j]);
+    for (u32 j = 0; j < 4; j++) tmem_ld16(src + 16u * j, v[j]);
     tmem_wait_ld();
     float acc = 0.0f;
 #pragma unroll
@@ -302,149 +315,183 @@ __device__ __forceinline__ float infer_epi2(u32 tacc, u32 lane_base, u32 c0, con
             const u32 c = c0 + 16u * j + t;
             const float4 bb = *reinterpret_cast<const float4 *>(bias.b2 + c);
             const float4 ww = *reinterpret_cast<const float4 *>(bias.w3 + c);
-            acc = fmaf(bf16_round(fmaxf(__uint_as_float(v[j][t]) + bb.x, 0.0f)), ww.x, acc);
-            acc = fmaf(bf16_round(fmaxf(__uint_as_float(v[j][t + 1]) + bb.y, 0.0f)), ww.y, acc);
-            acc = fmaf(bf16_round(fmaxf(__uint_as_float(v[j][t + 2]) + bb.z, 0.0f)), ww.z, acc);
-            acc = fmaf(bf16_round(fmaxf(__uint_as_float(v[j][t + 3]) + bb.w, 0.0f)), ww.w, acc);
+            const u32 h0 = relu_bf16x2(__uint_as_float(v[j][t]) + bb.x, __uint_as_float(v[j][t + 1]) + bb.y);
+            const u32 h1 = relu_bf16x2(__uint_as_float(v[j][t + 2]) + bb.z, __uint_as_float(v[j][t + 3]) + bb.w);
+            acc = fmaf(__uint_as_float(h0 << 16), ww.x, acc);
+            acc = fmaf(__uint_as_float(h0 & 0xffff0000u), ww.y, acc);
+            acc = fmaf(__uint_as_float(h1 << 16), ww.z, acc);
+            acc = fmaf(__uint_as_float(h1 & 0xffff0000u), ww.w, acc);
         }
     }
     return acc;
 }
 
-__global__ void __launch_bounds__(kInferThreads, 1)
+// The mbarriers of mlp_infer_kernel: layer-1 halves and layer 2 done (committed by the MMAs), activation halves,
+// one-hot tile and layer-2 accumulators handed over (one arrival per epilogue warp), and the final one.
+enum { kBarL1a, kBarL1b, kBarL2, kBarE1a, kBarE1b, kBarX, kBarE2, kBarEnd, kBarCount };
+
+__global__ void __launch_bounds__(kInferBlock, 1)
     mlp_infer_kernel(const u64 *__restrict__ kmers, u64 n, u32 k, const bf16 *__restrict__ W1b,
                      const bf16 *__restrict__ W2b, const InferBias bias, const InferOut out, int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bar1, bar2;
+    __shared__ uint64_t bar[kBarCount];
     __shared__ u32 tmem_s;
     uint8_t *sW1 = smem;
     uint8_t *sW2 = smem + kHid * kIn * 2;
     uint8_t *sX = sW2 + kHid * kHid * 2;
-    float *sRed = reinterpret_cast<float *>(sX + kTileM * kIn * 2);  // [kColGroups][kTileM] partial dots
+    float *sRed = reinterpret_cast<float *>(sX + kTileM * kIn * 2);  // [kColGroups - 1][kTileM] partial dots
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const u32 quarter = warp & 3u, cg = warp >> 2;
-    const u32 trow = quarter * 32u + lane;  // this thread's row of the tile
-    const u32 c0 = cg * kGroupCols;         // its first hidden column
-    const u32 xr = tid & (kTileM - 1u), xg = tid / kTileM;  // one-hot: row, chunk group
-    constexpr u32 kChunks = kIn / 8 / kColGroups;             // 4 of the 16 chunks of a row
     // weights into the canonical K-major layouts (once per launch)
-    for (u32 i = tid; i < kHid * (kIn / 8); i += kInferThreads) {
+    for (u32 i = tid; i < kHid * (kIn / 8); i += kInferBlock) {
         const u32 r = i / (kIn / 8), kc = i % (kIn / 8);
         *reinterpret_cast<uint4 *>(sW1 + canon_offset(kHid, r, kc * 8)) =
             *reinterpret_cast<const uint4 *>(W1b + (size_t)r * kIn + kc * 8);
     }
-    for (u32 i = tid; i < kHid * (kHid / 8); i += kInferThreads) {
+    for (u32 i = tid; i < kHid * (kHid / 8); i += kInferBlock) {
         const u32 r = i / (kHid / 8), kc = i % (kHid / 8);
         *reinterpret_cast<uint4 *>(sW2 + canon_offset(kHid, r, kc * 8)) =
             *reinterpret_cast<const uint4 *>(W2b + (size_t)r * kHid + kc * 8);
     }
     if (warp == 0) tmem_alloc(&tmem_s, 512);
     if (tid == 0) {
-        mbar_init(&bar1, 1);
-        mbar_init(&bar2, 1);
-    }
-    // the first tile's one-hot tile
-    u64 tile = blockIdx.x;
-    {
-        const u64 row = tile * kTileM + xr;
-        onehot_chunks(sX, kTileM, xr, row < n ? kmers[row] : 0ull, k, xg * kChunks, (xg + 1) * kChunks);
+        for (u32 i = 0; i < kBarCount; i++)
+            mbar_init(&bar[i], i >= kBarE1a && i <= kBarE2 ? kInferThreads / 32u : 1u);
     }
     fence_smem_to_async();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
     const u32 T0 = tmem_s;
-    const u32 lane_base = (quarter * 32u) << 16;
-    const float bias3 = bias.b3;
-    auto mma1 = [&](u32 tacc) {  // layer 1: one-hot tile x W1^T into tacc (thread 0, after a thread sync)
-        fence_after_sync();
-#pragma unroll
-        for (u32 s = 0; s < kIn / 16; s++) {
-            const u64 da = smem_desc(smem_addr(sX) + s * 2u * kTileM * 16u, kTileM * 16u, 128u);
-            const u64 db = smem_desc(smem_addr(sW1) + s * 2u * kHid * 16u, kHid * 16u, 128u);
-            mma_ss(tacc, da, db, idesc_bf16(kTileM, kHid), s > 0);
-        }
-        mma_commit(&bar1);
+    // a warp's wait: all lanes see the phase, or the warp leaves its loop
+    auto wait = [&](u32 b, u32 parity, int code) {
+        return __all_sync(0xffffffffu, mbar_wait(&bar[b], parity, err, code));
     };
-    u32 ph1 = 0, ph2 = 0;
-    bool pend1 = false, pend2 = false;  // an MMA commit outstanding on bar1 / bar2
-    bool ok = true;
-    u32 half = 0;  // this tile accumulates in columns [256 half, +256), its A2 at the other half
-    if (tid == 0) mma1(T0);
-    pend1 = true;
-    for (;;) {
-        const u32 tacc = T0 + 256u * half, ta2 = T0 + 256u * (half ^ 1u);
-        // ---- layer 1 done: bias, ReLU, BF16 into the other half's first 128 columns
-        bool got = mbar_wait(&bar1, ph1, err, kErrInferWait1);
-        ph1 ^= 1u;
-        pend1 = false;
-        fence_after_sync();
-        if (!__syncthreads_and(got)) { ok = false; break; }
-        infer_epi1(tacc, ta2, lane_base, c0, bias);
-        fence_before_sync();
-        __syncthreads();
-        if (tid == 0) {
+    auto region = [&](u32 i) { return T0 + (i & 3u) * 128u; };
+    if (warp < kInferThreads / 32u) {
+        // ---- epilogue warps
+        const u32 wu = __shfl_sync(0xffffffffu, warp, 0);  // the warp's number as a uniform value
+        const u32 quarter = wu & 3u, cg = wu >> 2, trow = quarter * 32u + lane;
+        const u32 lane_base = (quarter * 32u) << 16;
+        const u32 xr = tid & (kTileM - 1u), xg = tid / kTileM;     // one-hot: row, chunk group
+        constexpr u32 kChunks = kIn / 8 / kColGroups;                // 4 of the 16 chunks of a row
+        auto arrive = [&](u32 b) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar[b]);
+        };
+        auto one_hot = [&](u64 kmer) {
+            onehot_chunks(sX, kTileM, xr, kmer, k, xg * kChunks, (xg + 1) * kChunks);
+            fence_smem_to_async();
+            arrive(kBarX);
+        };
+        u64 tile = blockIdx.x;
+        one_hot(tile * kTileM + xr < n ? kmers[tile * kTileM + xr] : 0ull);
+        for (u32 it = 0;; it++) {
+            const u32 ph = it & 1u;
+            const u64 next = tile + gridDim.x;
+            const bool has_next = next * kTileM < n;
+            const u64 kmer = has_next && next * kTileM + xr < n ? __ldg(kmers + next * kTileM + xr) : 0ull;
+            const u32 a2 = region(it + 2u) + lane_base + cg * 16u;
+            // layer 1, bias, ReLU, BF16: this warp's 32 columns of each half
+            if (!wait(kBarL1a, ph, kErrInferWait1)) break;
             fence_after_sync();
+            infer_epi1<32>(region(it) + lane_base + cg * 32u, a2, cg * 32u, bias);
+            fence_before_sync();
+            arrive(kBarE1a);
+            if (!wait(kBarL1b, ph, kErrInferWait1)) break;
+            fence_after_sync();
+            infer_epi1<32>(region(it + 1u) + lane_base + cg * 32u, a2 + 64u, 128u + cg * 32u, bias);
+            fence_before_sync();
+            arrive(kBarE1b);
+            if (has_next) one_hot(kmer);  // layer 1 has read this tile's
+            // layer 2: this warp's 64 columns
+            if (!wait(kBarL2, ph, kErrInferWait2)) break;
+            fence_after_sync();
+            const float dot = infer_epi2(region(cg < 2u ? it + 3u : it) + lane_base + (cg & 1u) * 64u, cg * kGroupCols, bias);
+            if (cg) sRed[(cg - 1u) * kTileM + trow] = dot;
+            fence_before_sync();
+            arrive(kBarE2);
+            // all accumulators are read (the next activations go over them) and all partial dots written; they are
+            // written again only after the next layer 2, which waits for every warp's next activations
+            if (!wait(kBarE2, ph, kErrInferWait2)) break;
+            fence_after_sync();
+            if (cg == 0) {
+                const u64 row = tile * kTileM + trow;
+                float sum = dot;
 #pragma unroll
-            for (u32 s = 0; s < kHid / 16; s++) {
-                const u64 db = smem_desc(smem_addr(sW2) + s * 2u * kHid * 16u, kHid * 16u, 128u);
-                mma_ts(tacc, ta2 + s * 8u, db, idesc_bf16(kTileM, kHid), s > 0);
+                for (u32 g = 0; g + 1u < kColGroups; g++) sum += sRed[g * kTileM + trow];
+                const float lg = sum + bias.b3;
+                if (out.logits && row < n) out.logits[row] = lg;
+                if (out.reject) {
+                    // the sandwich's decision: rejected by the model at tau and by the backup Bloom filter
+                    const Bloom bloom{out.bloom_bits, out.bloom_mask, out.bloom_hashes};
+                    const bool rej = row < n && lg < out.tau && !bloom.probe(kmer_key(kmers[row], k));
+                    const u32 bits = __ballot_sync(0xffffffffu, rej);
+                    const u64 first = tile * kTileM + quarter * 32u;  // this warp's 32 rows
+                    if (lane == 0 && first < n) out.reject[first >> 5] = bits;
+                }
             }
-            mma_commit(&bar2);
+            if (!has_next) break;
+            tile = next;
         }
-        pend2 = true;
-        // ---- while layer 2 runs: the next tile's one-hot tile (layer 1 has read this one)
-        const u64 next = tile + gridDim.x;
-        const bool has_next = next * kTileM < n;
-        if (has_next) {
-            const u64 row = next * kTileM + xr;
-            onehot_chunks(sX, kTileM, xr, row < n ? kmers[row] : 0ull, k, xg * kChunks, (xg + 1) * kChunks);
-        }
-        fence_smem_to_async();
-        got = mbar_wait(&bar2, ph2, err, kErrInferWait2);
-        ph2 ^= 1u;
-        pend2 = false;
-        fence_after_sync();
-        if (!__syncthreads_and(got)) { ok = false; break; }
-        // ---- layer 2 done: the next tile's layer 1 into the other half (this tile's A2 is spent)
-        if (has_next) {
-            if (tid == 0) mma1(ta2);
-            pend1 = true;
-        }
-        // ---- this tile's layer-2 epilogue while the next tile's layer 1 runs
-        sRed[cg * kTileM + trow] = infer_epi2(tacc, lane_base, c0, bias);
-        fence_before_sync();
-        __syncthreads();
-        if (cg == 0) {
-            const u64 row = tile * kTileM + trow;
-            float sum = 0.0f;
+    } else {
+        // ---- MMA warp: one lane issues
+        constexpr u32 idesc = idesc_bf16(kTileM, 128);
+        constexpr u32 half_rows = 128u / 8u * 128u;  // byte offset of rows 128.. of a weight tile
+        auto layer1 = [&](u32 half, u32 dst) {
 #pragma unroll
-            for (u32 g = 0; g < kColGroups; g++) sum += sRed[g * kTileM + trow];
-            const float lg = sum + bias3;
-            if (out.logits && row < n) out.logits[row] = lg;
-            if (out.reject) {
-                // the sandwich's decision: rejected by the model at tau and by the backup Bloom filter
-                const Bloom bloom{out.bloom_bits, out.bloom_mask, out.bloom_hashes};
-                const bool rej = row < n && lg < out.tau && !bloom.probe(kmer_key(kmers[row], k));
-                const u32 bits = __ballot_sync(0xffffffffu, rej);
-                const u64 first = tile * kTileM + quarter * 32u;  // this warp's 32 rows
-                if (lane == 0 && first < n) out.reject[first >> 5] = bits;
+            for (u32 s = 0; s < kIn / 16; s++) {
+                const u64 da = smem_desc(smem_addr(sX) + s * 2u * kTileM * 16u, kTileM * 16u, 128u);
+                const u64 db = smem_desc(smem_addr(sW1) + s * 2u * kHid * 16u + half * half_rows, kHid * 16u, 128u);
+                mma_ss(dst, da, db, idesc, s > 0);
             }
-        }
-        // sRed is reused and this half's columns take the next tile's A2 only after every thread is here
-        __syncthreads();
+            mma_commit(&bar[half ? kBarL1b : kBarL1a]);
+        };
+        // layer 2 over the activations 128 kh .. +127, both halves of its columns
+        auto layer2 = [&](u32 kh, u32 a2, u32 lo, u32 hi) {
+#pragma unroll
+            for (u32 s = 8u * kh; s < 8u * kh + 8u; s++) {
+                const u32 b = smem_addr(sW2) + s * 2u * kHid * 16u;
+                mma_ts(lo, a2 + s * 8u, smem_desc(b, kHid * 16u, 128u), idesc, s > 0);
+                mma_ts(hi, a2 + s * 8u, smem_desc(b + half_rows, kHid * 16u, 128u), idesc, s > 0);
+            }
+        };
+        bool ok = wait(kBarX, 0, kErrInferWait1);
         fence_after_sync();
-        if (!has_next) break;
-        tile = next;
-        half ^= 1u;
-    }
-    if (!ok && tid == 0) {  // let the MMAs still in flight land before the columns are freed
-        if (pend1) mbar_wait(&bar1, ph1, err, kErrInferWait1);
-        if (pend2) mbar_wait(&bar2, ph2, err, kErrInferWait2);
+        if (ok && lane == 0) {
+            layer1(0, region(0));
+            layer1(1, region(1));
+        }
+        u64 tile = blockIdx.x;
+        for (u32 it = 0; ok; it++) {
+            const u32 ph = it & 1u, a2 = region(it + 2u), lo = region(it + 3u), hi = region(it);
+            if (!(ok = wait(kBarE1a, ph, kErrInferWait1))) break;
+            fence_after_sync();
+            if (lane == 0) layer2(0, a2, lo, hi);
+            if (!(ok = wait(kBarE1b, ph, kErrInferWait1))) break;
+            fence_after_sync();
+            if (lane == 0) {
+                layer2(1, a2, lo, hi);
+                mma_commit(&bar[kBarL2]);
+            }
+            tile += gridDim.x;
+            if (tile * kTileM >= n) break;
+            if (!(ok = wait(kBarX, ph ^ 1u, kErrInferWait1))) break;
+            fence_after_sync();
+            if (lane == 0) layer1(0, region(it + 1u));  // over the second half of layer 1, which E1b handed over
+            if (!(ok = wait(kBarL2, ph, kErrInferWait2))) break;
+            fence_after_sync();
+            if (lane == 0) layer1(1, region(it + 2u));  // over the activations, which layer 2 has read
+        }
+        // every MMA has landed before the columns are freed
+        if (lane == 0) {
+            mma_commit(&bar[kBarEnd]);
+            mbar_wait(&bar[kBarEnd], 0, err, kErrInferWait2);
+        }
+        __syncwarp();
     }
     fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_s, 512);
+    if (warp == 0) tmem_dealloc(T0, 512);
 }
 
 // ------------------------------------------------------- training helpers
@@ -697,7 +744,7 @@ int infer(const u64 *kmers, u64 n, u32 k, const bf16 *W1b, const bf16 *W2b, cons
     }
     const u64 tiles = (n + kTileM - 1) / kTileM;
     const u32 grid = (u32)std::min<u64>(tiles, (u64)num_sms);
-    mlp_infer_kernel<<<grid, kInferThreads, kInferSmem, s>>>(kmers, n, k, W1b, W2b, bias, out, err);
+    mlp_infer_kernel<<<grid, kInferBlock, kInferSmem, s>>>(kmers, n, k, W1b, W2b, bias, out, err);
     SBWT_CHECK_CUDA(cudaGetLastError());
     return 0;
 }

@@ -51,6 +51,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, u32 parity) {
     return ok != 0;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
 // Waits for phase `parity` of the barrier; on timeout sets *err = code and
 // returns false (the caller skips the rest of its work).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, u32 parity, int *err, int code) {
