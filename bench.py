@@ -79,7 +79,7 @@ def parse():
                     help="skip the batched and pangenome workloads measured beside the headline")
     ap.add_argument("--workload-steps", type=int, default=3, help="timed steps of each workload beside the headline")
     ap.add_argument("--search-mode", choices=["every", "skip", "stream"], default="stream",
-                    help="main leg: every k-mer searched (as the reference), absent-run skip, or skip + backward steps")
+                    help="main leg: every k-mer searched (as the reference), absent-run skip, or the forward walk along the graph's paths")
     ap.add_argument("--pf-queries", type=int, default=200_000_000)
     ap.add_argument("--pf-steps", type=int, default=20000)
     ap.add_argument("--workload", choices=["large", "batched", "pangenome"], default="large",
@@ -284,13 +284,13 @@ def cpu_reference(ox, letters, rows, k, p, budget_s, table):
 
 
 def walk_model(ans, steps, rows, k, p, stream, max_rows=20000):
-    """How the run walk settles the k-mers of the first `max_rows` reads, from per-k-mer oracle answers
-    and step counts (right to left per read; a search that fails after m letters settles k-m+1
-    k-mers; with `stream`, the k-mer left of a found one takes a backward step): the share of k-mers
-    searched from scratch, the share reached by a backward step, and the mean rank-pair steps of a
-    search from scratch."""
+    """How the walk settles the k-mers of the first `max_rows` reads, from per-k-mer oracle answers and
+    step counts: the share of k-mers searched from scratch, the share reached along a path, and the
+    mean rank-pair steps of a search from scratch.  Without `stream`: right to left per read, a search
+    that fails after m letters settles k-m+1 k-mers.  With `stream`: one search per stretch of
+    consecutive present k-mers, the rest of the stretch along the path, no rank-pair steps."""
     import oracle as orc
-    searched = back = total = walk_steps = 0
+    searched = path = total = walk_steps = 0
     j0 = 0
     for r in range(min(rows.size - 1, max_rows)):
         n = int(rows[r + 1] - rows[r]) - k + 1
@@ -298,38 +298,34 @@ def walk_model(ans, steps, rows, k, p, stream, max_rows=20000):
             continue
         if j0 + n > ans.size:
             break
-        j = j0 + n - 1
-        have = False
-        while j >= j0:
-            hit = ans[j] != orc.NOT_FOUND
-            if stream and have:
-                back += 1
-                have = hit
-                j -= 1
-            else:
+        if stream:
+            hit = ans[j0:j0 + n] != orc.NOT_FOUND
+            starts = int(hit[0]) + int((hit[1:] & ~hit[:-1]).sum())
+            searched += starts
+            path += int(hit.sum()) - starts
+        else:
+            j = j0 + n - 1
+            while j >= j0:
                 searched += 1
                 walk_steps += int(steps[j])
-                if hit:
-                    have = True
-                    j -= 1
-                else:
-                    j -= k - min(max(p, p + int(steps[j])), k) + 1
+                j -= 1 if ans[j] != orc.NOT_FOUND else k - min(max(p, p + int(steps[j])), k) + 1
         j0 += n
         total += n
-    return searched / max(total, 1), back / max(total, 1), walk_steps / max(searched, 1)
+    return searched / max(total, 1), path / max(total, 1), walk_steps / max(searched, 1)
 
 
 SECTOR = 32  # bytes: the unit in which L2 misses are filled from DRAM
 
 
-def dram_model(n_kmers, n_letters, n_rows, searched, back, walk_steps, sizes, l2_bytes, answers=True):
-    """Algorithmic DRAM bytes per k-mer of one launch of the run-walking search kernel.
+def dram_model(n_kmers, n_letters, n_rows, searched, path, walk_steps, sizes, l2_bytes, answers=True):
+    """Algorithmic DRAM bytes per k-mer of one search of a batch of reads.
     Compulsory streams: packed letters (2 bits per letter), the row table (row start + first k-mer
     index, 16 B per row), the u64 answers (8 B, written once) and the membership bitmap (1 bit).
-    Gathers: one presearch entry per search from scratch, one backward-table entry per backward
-    step, and two 32-byte lines per rank-pair step (one when the interval is a single node; two is
-    the bound), each a 32-byte sector from DRAM when its table cannot stay in L2 (larger than half
-    of it) and L2 traffic otherwise."""
+    Gathers: one presearch entry per search from scratch; in the forward walk also one label and one
+    path position per search and four bytes of the path's nodes per present k-mer; in the
+    absent-run skip two 32-byte lines per rank-pair step (one when the interval is a single node; two
+    is the bound).  Each is a 32-byte sector (the nodes: their four bytes) from DRAM when its table
+    cannot stay in L2 (larger than half of it) and L2 traffic otherwise."""
     per = {
         "letters": n_letters / 4.0 / n_kmers,
         "row_table": 16.0 * n_rows / n_kmers,
@@ -337,16 +333,15 @@ def dram_model(n_kmers, n_letters, n_rows, searched, back, walk_steps, sizes, l2
         "bitmap": 0.125,
     }
     gathers = {
-        "presearch": (searched, sizes["presearch"]),
-        "backward_table": (back, sizes["backward_table"]),
-        "lines": (searched * walk_steps * 2.0, sizes["lines"]),
+        "presearch": (searched * SECTOR, sizes["presearch"]),
+        "labels": (searched * SECTOR if sizes["labels"] else 0.0, sizes["labels"]),
+        "node_pos": (searched * SECTOR if sizes["node_pos"] else 0.0, sizes["node_pos"]),
+        "path_node": ((searched + path) * 4.0 if sizes["path_node"] and answers else 0.0, sizes["path_node"]),
+        "lines": (searched * walk_steps * 2.0 * SECTOR, sizes["lines"]),
     }
     l2 = {}
-    for name, (count, table_bytes) in gathers.items():
-        if table_bytes > l2_bytes / 2:
-            per[name] = count * SECTOR
-        else:
-            l2[name] = count * SECTOR
+    for name, (table_traffic, table_bytes) in gathers.items():
+        (per if table_bytes > l2_bytes / 2 else l2)[name] = table_traffic
     return sum(per.values()), per, l2
 
 
@@ -383,15 +378,18 @@ def kernel_traffic(kernel, workload, n_kmers):
 
 
 def table_sizes(n_columns, p, stream_tables=True):
-    """Bytes of the index structures the run walk gathers from: presearch table (8-byte entries below
-    2^32 columns), backward table (8 bytes per column) and the 32-byte lines of the four vectors."""
+    """Bytes of the index structures the walk gathers from: presearch table (8-byte entries below 2^32
+    columns), the forward walk's sorted labels (8 bytes per column), path positions and path nodes (4
+    bytes each), and the 32-byte lines of the four vectors."""
     lpc = (n_columns // 224 + 1 + 7) // 8 * 8
     return {"presearch": (1 << (2 * p)) * (8 if n_columns < (1 << 32) else 16) if p else 0,
-            "backward_table": 8 * n_columns if stream_tables else 0,
+            "labels": 8 * n_columns if stream_tables else 0,
+            "node_pos": 4 * n_columns if stream_tables else 0,
+            "path_node": 4 * n_columns if stream_tables else 0,
             "lines": 4 * lpc * 32}
 
 
-def roofline(kernel, kern_ms, n_kmers, n_letters, n_rows, n_columns, p, searched, back, walk_steps, mean_steps,
+def roofline(kernel, kern_ms, n_kmers, n_letters, n_rows, n_columns, p, searched, path, walk_steps, mean_steps,
              p_steps, dev, peak, peak_kind, traffic_workload, stream_tables=True, answers=True):
     """The `roofline` object of the dominant kernel: walk-aware algorithmic DRAM bytes (dram_model)
     over the kernel's CUDA-event time, against the measured copy bandwidth; the measured DRAM traffic
@@ -400,7 +398,7 @@ def roofline(kernel, kern_ms, n_kmers, n_letters, n_rows, n_columns, p, searched
     import torch
     l2_bytes = torch.cuda.get_device_properties(dev).L2_cache_size
     sizes = table_sizes(n_columns, p, stream_tables)
-    b_kmer, parts, l2 = dram_model(n_kmers, n_letters, n_rows, searched, back, walk_steps, sizes, l2_bytes, answers)
+    b_kmer, parts, l2 = dram_model(n_kmers, n_letters, n_rows, searched, path, walk_steps, sizes, l2_bytes, answers)
     secs = kern_ms / 1e3
     achieved = n_kmers * b_kmer / secs / 1e9
     traffic, tr = kernel_traffic(kernel, traffic_workload, n_kmers)
@@ -411,7 +409,7 @@ def roofline(kernel, kern_ms, n_kmers, n_letters, n_rows, n_columns, p, searched
             "bytes_per_kmer_parts": {kk: round(vv, 4) for kk, vv in parts.items()},
             "l2_bytes_per_kmer": {kk: round(vv, 4) for kk, vv in l2.items()},
             "table_bytes": sizes, "l2_cache_bytes": l2_bytes,
-            "searched_fraction": searched, "backward_step_fraction": back,
+            "searched_fraction": searched, "path_fraction": path,
             "steps_per_search": walk_steps, "steps_counted_at_p": p_steps,
             "traffic_per_kmer": traffic / n_kmers if traffic else None,
             "traffic_over_model": traffic / (n_kmers * b_kmer) if traffic else None,
@@ -501,7 +499,7 @@ def timed_search(ix, step, steps, warmup, dev, stream, world=1):
 
 def oracle_check(orc, paths, letters, rows, k, p, seconds, got_fn, stream_mode, runs_form):
     """Answers of a bounded prefix of the batch from the oracle (C restatement of the reference search), compared
-    with the device answers; the walk model of the run walk from the same sample."""
+    with the device answers; the walk model from the same sample."""
     ox = orc.OracleIndex.from_files(paths)
     p_cpu = min(p, 12)  # answers do not depend on p; a CPU table beyond 4^12 entries costs minutes
     table = ox.presearch(p_cpu) if p_cpu else None
@@ -510,10 +508,10 @@ def oracle_check(orc, paths, letters, rows, k, p, seconds, got_fn, stream_mode, 
     if not np.array_equal(got, ans):
         raise SystemExit(f"bench: {int((got != ans).sum())} of {ans.size} sampled answers differ from the oracle")
     mean_steps = float(steps.mean())
-    searched, back, walk_steps = (walk_model(ans, steps, rows, k, p_cpu, stream_mode) if runs_form
+    searched, path, walk_steps = (walk_model(ans, steps, rows, k, p_cpu, stream_mode) if runs_form
                                   else (1.0, 0.0, mean_steps))
     return {"rate": rate, "ans": ans, "nr": nr, "threads": threads, "p_cpu": p_cpu, "mean_steps": mean_steps,
-            "searched": searched, "back": back, "walk_steps": walk_steps}
+            "searched": searched, "path": path, "walk_steps": walk_steps}
 
 
 def main():
@@ -550,15 +548,15 @@ def main():
         search_mode=MODES[args.search_mode])
     del seqs
     runs_form = args.kpt == 0 and args.search_mode != "every" and (args.tpk <= 1 or args.layout == "poppy")
-    kernel = ("search_runs_kernel" + ("<stream>" if args.search_mode == "stream" else "<skip>") if runs_form
-              else ("search_queue_kernel" if args.kpt == 0 else "search_kernel"))
+    kernel = ("walk_kernel" if args.search_mode == "stream" else "search_runs_kernel<skip>") if runs_form else (
+        "search_queue_kernel" if args.kpt == 0 else "search_kernel")
     if args.l2_fetch:
         ix.set_l2_fetch_granularity(args.l2_fetch)
     if args.window or args.evict >= 0 or args.l2_persist >= 0 or args.blocks_per_sm:
         ix.set_walk_options(window=args.window or None, evict=args.evict if args.evict >= 0 else None,
                             l2_persist=args.l2_persist if args.l2_persist >= 0 else None,
                             blocks_per_sm=args.blocks_per_sm or None)
-    build_times = ix.build_times()  # device ms: rank words (lines), poppy, presearch, backward table
+    build_times = ix.build_times()  # device ms: rank words (lines), poppy, presearch, walk structures
     info = ix.info()
 
     d_letters = torch.from_numpy(letters).to(dev)
@@ -616,7 +614,7 @@ def main():
         member_only = {"value": n_kmers * args.steps / (tt / 1e3), "ms_per_step": tt / args.steps,
                        "search_kernel_ms": km, "output": "membership bitmap only (no answers)",
                        "roofline": roofline(kernel, km, n_kmers, letters.size, rows.size - 1, info["n_bits"], p,
-                                            chk["searched"], chk["back"], chk["walk_steps"], chk["mean_steps"],
+                                            chk["searched"], chk["path"], chk["walk_steps"], chk["mean_steps"],
                                             chk["p_cpu"], dev, *measured_hbm(), None,
                                             stream_tables=args.search_mode == "stream", answers=False)}
         del d_mem2
@@ -628,7 +626,7 @@ def main():
     if rank == 0:
         peak, peak_kind = measured_hbm()
         roof = roofline(kernel, kern_ms, n_kmers, letters.size, rows.size - 1, info["n_bits"], p, chk["searched"],
-                        chk["back"], chk["walk_steps"], chk["mean_steps"], chk["p_cpu"], dev, peak, peak_kind,
+                        chk["path"], chk["walk_steps"], chk["mean_steps"], chk["p_cpu"], dev, peak, peak_kind,
                         args.workload if args.scale == 1.0 and args.query_scale == 1.0 else None,
                         stream_tables=args.search_mode == "stream")
         hits = int((d_ans.cpu().numpy().view(np.uint64) != orc.NOT_FOUND).sum())
@@ -811,7 +809,7 @@ def device_leg(ix, sg, orc, paths, letters, rows, k, p, steps, warmup, dev, stre
            "bit_exact_sample": {"kmers": int(chk["ans"].size), "equal": True},
            "gpu_launches": launches * steps, "clocks": clk,
            "roofline": roofline(kernel, km, n_kmers, letters.size, rows.size - 1, info["n_bits"], p, chk["searched"],
-                                chk["back"], chk["walk_steps"], chk["mean_steps"], chk["p_cpu"], dev, peak,
+                                chk["path"], chk["walk_steps"], chk["mean_steps"], chk["p_cpu"], dev, peak,
                                 peak_kind, workload_key)}
     del d_letters, d_rows, d_ans, d_mem
     torch.cuda.empty_cache()
@@ -884,7 +882,7 @@ def other_workloads(args, sg, orc, k, dev, stream, rank, world, local_rank):
     letters, rows = batched_queries(args, rank)
     ix, paths, _, _ = open_index(sg, [small], k, 10, args, rank, 1, local_rank, "small",
                                  search_mode=sg.SEARCH_STREAM)
-    kern = "search_runs_kernel<stream>"
+    kern = "walk_kernel"
     out["batched"] = device_leg(ix, sg, orc, paths, letters, rows, k, 10, steps, 2, dev, stream, kern,
                                 "batched" if args.scale == 1.0 else None, min(args.cpu_seconds, 4.0),
                                 WORKLOADS["batched"])

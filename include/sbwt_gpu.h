@@ -74,11 +74,14 @@ typedef struct {
  * SKIP_ABSENT: each read is walked from right to left; when a k-mer's search
  *   fails after m letters, those m letters are in no indexed k-mer, so the
  *   k-m+1 k-mers containing them are answered absent without a search.
- * STREAM: SKIP_ABSENT, and after a k-mer is found the k-mer one letter to its
- *   left is reached by one backward step (one load from a per-column table
- *   of predecessor groups) instead of a new search.  Needs the line layout's
- *   index size limit and about 8.6 bytes per column, built on the GPU when
- *   the mode is selected. */
+ * STREAM: each read is walked from left to right along the paths of the
+ *   graph: an absent stretch is found in a bitmap of the substrings of q
+ *   letters, a present k-mer by a search in the sorted labels, and the k-mers
+ *   behind it by comparing the read with the path's text.  Serves every
+ *   layout of an index within the line layout's size limit, and needs about
+ *   17.2 bytes per column and the bitmap (at most 32 MiB up to 4^14 columns),
+ *   built on the GPU when the mode is selected.  Lists of single k-mers are
+ *   searched through the same structures. */
 #define SBWT_SEARCH_EVERY_KMER 0
 #define SBWT_SEARCH_SKIP_ABSENT 1
 #define SBWT_SEARCH_STREAM 2
@@ -124,7 +127,7 @@ int sbwt_presearch(sbwt_index *index, uint32_t p);
 
 /* Device time in ms of the index's last build phases: ms[0] the line layout
  * (rank words), ms[1] the poppy L0/L12 structures (0 if not built), ms[2]
- * the presearch table (its last build), ms[3] the backward-step structures.
+ * the presearch table (its last build), ms[3] the structures of SBWT_SEARCH_STREAM.
  * The reference prints its presearch time (include/matrix_sbwt.hpp:188) and
  * builds its rank structures on the CPU (rank_data_structures.hpp:142-198). */
 int sbwt_build_times(const sbwt_index *index, float ms[4]);
@@ -152,10 +155,10 @@ int sbwt_configure(sbwt_index *index, int32_t layout, uint32_t bits_in_superbloc
                    int32_t with_shuffles, uint32_t kmers_per_thread, uint32_t threads_per_kmer,
                    uint32_t threads_per_block);
 
-/* Knobs of the run walk (searches of reads), each SBWT_KEEP to leave it:
+/* Knobs of the walks (searches of reads), each SBWT_KEEP to leave it:
  * window = k-mers per window of the work split (64, 128, 256; line layout),
  * blocks_per_sm = resident blocks per SM of the persistent grid (0: as many
- * as fit), evict = the L2 policy of the presearch and backward-table gathers
+ * as fit), evict = the L2 policy of the presearch gathers
  * (0: evict-first when the table exceeds half of L2, 1: never, 2: always),
  * l2_persist = hold the rank lines in the persisting L2 set-aside (1) or not
  * (0).  The autotuner sets them; the answers do not depend on them.  No
@@ -164,7 +167,7 @@ int sbwt_set_walk_options(sbwt_index *index, uint32_t window, uint32_t blocks_pe
                           int32_t l2_persist);
 
 /* Selects the search mode (SBWT_SEARCH_*) for later searches of reads on this
- * index, building the backward-step structures on first use of
+ * index, building its structures on first use of
  * SBWT_SEARCH_STREAM.  No reference counterpart: the reference searches every
  * k-mer (include/gpu/search_kernel.hpp:61-104). */
 int sbwt_set_search_mode(sbwt_index *index, int32_t mode);

@@ -146,7 +146,7 @@ class Index:
                                  kmers_per_thread, threads_per_kmer, threads_per_block))
 
     def build_times(self):
-        """Device ms of the last build phases: lines, poppy, presearch table, backward-step structures."""
+        """Device ms of the last build phases: lines, poppy, presearch table, the structures of SBWT_SEARCH_STREAM."""
         ms = (ctypes.c_float * 4)()
         check(lib.sbwt_build_times(self._h, ms))
         return {"lines_ms": ms[0], "poppy_ms": ms[1], "presearch_ms": ms[2], "backward_ms": ms[3]}

@@ -14,9 +14,8 @@
 //      {128,256});
 //   2. the run walk's knobs on the best layout, one at a time, each kept
 //      when it is faster: window (64 / 256 k-mers against 128), resident
-//      blocks per SM, the evict-first policy of the presearch and
-//      backward-table gathers (never / always against by table size), the
-//      rank lines held in the persisting L2 set-aside, and the compact
+//      blocks per SM, the evict-first policy of the presearch gathers
+//      (never / always against by table size), the rank lines held in the persisting L2 set-aside, and the compact
 //      4-byte presearch entries;
 //   3. with SBWT_TUNE_P the presearch depth p in {8,10,12,14,15} (p <= k),
 //      then the window and the evict policy again at the chosen p.

@@ -39,9 +39,8 @@ constexpr u32 kMaxLinesPerChar = 1u << 24;  // 32-bit counts: 224 * 2^24 < 2^32
 #endif
 
 // Cache operator of the random gathers: SBWT_GATHER_CG = 1 reads the
-// presearch and backward-table entries with ld.global.cg (cached in L2
-// only), 2 also the rank lines; 0 reads them through the read-only L1 path
-// (ld.global.nc).
+// presearch entries with ld.global.cg (cached in L2 only), 2 also the rank
+// lines; 0 reads them through the read-only L1 path (ld.global.nc).
 #ifndef SBWT_GATHER_CG
 #define SBWT_GATHER_CG 0
 #endif
@@ -85,8 +84,7 @@ __device__ __forceinline__ u64 ld_nc(const u64 *p) {
     return v;
 }
 
-// Gathers with little reuse (a presearch entry, a backward-table entry) from
-// a table too large to stay in L2 are read with an L2 evict-first policy, so
+// Gathers with little reuse (a presearch entry) from a table too large to stay in L2 are read with an L2 evict-first policy, so
 // that they do not push the lines of the rank steps out of L2; gathers from a
 // table that fits use evict-normal (evict-first there makes them miss:
 // measured 28 % slower on an L2-resident index).  createpolicy and
@@ -128,19 +126,6 @@ __device__ __forceinline__ uint2 ld_gather_u32x2(const uint2 *p, bool ef, u64 po
     (void)ef;
     (void)pol;
     return __ldg(p);
-}
-
-__device__ __forceinline__ u64 ld_gather_u64(const u64 *p, bool ef, u64 pol) {
-#if SBWT_GATHER_EVICT_FIRST
-    if (ef) {
-        u64 v;
-        asm(SBWT_GATHER_LD ".L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(pol));
-        return v;
-    }
-#endif
-    (void)ef;
-    (void)pol;
-    return __ldg(reinterpret_cast<const unsigned long long *>(p));
 }
 
 // x >> s with the PTX rule that s >= 64 gives 0 (the reference relies on it,

@@ -48,9 +48,9 @@ struct SearchArgs {
     u32 found_only;               // with `walk`: answers of absent k-mers need not be written
     u32 piece;                    // with `walk`: k-mers per run at most
     u32 runs;                     // read mode: walk runs right to left with the absent-run skip
-    u32 stream;                   // with `runs`: backward steps from a found k-mer (needs sv)
+    u32 stream;                   // with `runs` and `reject`: backward steps from a found k-mer (needs sv)
     u32 index64;                  // with `runs`: the walk's 64-bit index form whatever the batch size
-    u32 ef_pre;                   // with `runs`: evict-first gathers from the presearch table (set when
+    u32 ef_pre;                   // with `runs` or `walk`: evict-first gathers from the presearch table (set when
                                   // it cannot stay in L2; device.cuh)
     u32 walk;                     // the searches of walk.cu, with wv and sv: the forward walk in read mode, else
                                   // the list search
@@ -151,7 +151,7 @@ struct sbwt_index {
     uint32_t *d_pre32 = nullptr;
     bool pre64 = false;
     int compact_pre = -1;  // the compact table: -1 = from SBWT_PRESEARCH_COMPACT, 0 = off, 1 = on
-    // backward-step structures (stream.cu): node nibbles, select samples
+    // structures of the backward step (stream.cu): node nibbles, select samples
     uint8_t *d_node = nullptr;
     uint32_t *d_sel = nullptr;
     // structures of the forward walk (WalkView, stream.cuh); walk_q = 0: not there
@@ -161,7 +161,7 @@ struct sbwt_index {
     uint32_t walk_q = 0;
     uint32_t sel_off[4] = {0, 0, 0, 0}, sel_n[4] = {0, 0, 0, 0};
     bool stream_ok = false;
-    // device ms of the last build of: lines, poppy, presearch table, backward-step structures
+    // device ms of the last build of: lines, poppy, presearch table, the walk's structures
     float build_ms[4] = {0, 0, 0, 0};
     // launch shape
     sbwt::KernelShape shape;
@@ -260,13 +260,13 @@ void l2_setaside_release(sbwt_index *ix);
 
 // search.cu
 int launch_search(const sbwt_index *ix, SearchArgs &a, cudaStream_t s, uint32_t *launched_blocks);
-// Evict-first policies for the run walk's gathers: a table gets one when it
+// Evict-first policy for the walks' presearch gathers: the table gets one when it
 // is larger than half of the device's L2 (it cannot stay there next to the
 // lines).
 void set_gather_policies(const sbwt_index *ix, SearchArgs &a);
 // Whether a batch of reads searched with the index's current shape and mode
-// runs the run-walking kernel (absent-run skip), and whether it also takes
-// backward steps.
+// walks its rows (absent-run skip), and whether it does so along the paths of
+// the graph (walk.cu; behind the learned prefilter by backward steps).
 bool runs_form(const sbwt_index *ix);
 bool stream_form(const sbwt_index *ix);
 // Work granularity of a launch: k-mers per grab, or for the run-walking form

@@ -1,11 +1,11 @@
 // packed_runs.cu -- the reference's kernel contract (sbwt_search_packed:
 // packed k-mer string + a positions array overwritten by the answers,
-// include/gpu/search_kernel.hpp:61-104) on the run-walking kernel.
+// include/gpu/search_kernel.hpp:61-104) on the walks of reads.
 //
 // K-mers whose positions follow each other (positions[j] = positions[j-1] + 1)
 // are consecutive windows of the packed string, so they form a run the walk
-// can take right to left with the absent-run skip and backward steps, whatever
-// the reads were; the reference's own positions (one run per read,
+// can take (walk.cu, or search.cu's absent-run skip), whatever the reads
+// were; the reference's own positions (one run per read,
 // include/gpu/positions_kernel.hpp:18-36) are of that kind.  The run starts
 // become a row table (first k-mer index and letter offset of each run), after
 // which the search is the one of sbwt_search_reads, writing its answers over

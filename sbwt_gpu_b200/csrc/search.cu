@@ -355,7 +355,12 @@ __global__ void __launch_bounds__(128, QueueMinBlocks<R>::value) search_queue_ke
 // k-mers at once and answers ~0 for all of them, so every answer equals the
 // reference's per-k-mer search.
 //
-// With STREAM, a found k-mer's node also gives the node of the k-mer one
+// Since the forward walk (walk.cu) took over the default mode, this kernel
+// serves SBWT_SEARCH_SKIP_ABSENT, k other than the index's, indexes without
+// the walk's structures, and with FILTER the reads behind the learned
+// prefilter, whose count of unsearched k-mers is defined by this order.
+//
+// With STREAM (FILTER only), a found k-mer's node also gives the node of the k-mer one
 // letter to its left by one backward step (stream.cuh) instead of a search
 // (presearch entry + k-p rank-pair steps); a failed backward step means that
 // k-mer is absent, and the next one is searched again.

@@ -1,6 +1,7 @@
-// stream.cu -- builds the backward-step structures (stream.cuh): select
-// samples, node nibbles and the backward table, on the GPU from the index's
-// lines alone, so that indexes loaded from the reference's files get them
+// stream.cu -- builds the walk's structures (stream.cuh): sorted labels, path
+// text, q-mer bitmap and group marks of the forward walk, select samples and
+// node nibbles of the backward step, on the GPU from the index's lines alone,
+// so that indexes loaded from the reference's files get them
 // too.  No reference counterpart.
 //
 // First letters and groups come from the labels: with pred(v) = the first
@@ -387,7 +388,7 @@ void free_walk(sbwt_index *ix) {
 
 int build_stream(sbwt_index *ix, cudaStream_t s) {
     if (ix->stream_ok) return 0;
-    if (!ix->lines_ok) return set_error("the backward step needs the line layout");
+    if (!ix->lines_ok) return set_error("the walk needs the line layout");
     if (ix->k > 32 || ix->k < 2) return set_error("k out of range");
     const u32 n = (u32)ix->n, k = ix->k;
     u64 total = 0;

@@ -1,5 +1,5 @@
-// stream.cuh -- select on the line layout and the backward step of the run
-// walk (device side).  No reference counterpart: the reference searches every
+// stream.cuh -- what the forward walk (walk.cu) reads beside the rank lines,
+// and the backward step of the prefiltered run walk (search.cu).  No reference counterpart: the reference searches every
 // k-mer from scratch (include/gpu/search_kernel.hpp:61-104).
 //
 // SBWT facts used (plain-matrix SBWT, nodes in colex order):
@@ -13,9 +13,8 @@
 // select_b(v - C[b]) whose first letter is a, if there is one.  Per node the
 // engine keeps four bits, two nodes per byte (even node in the low half): its
 // first letter (0 = $, 1..4 = A..T) and a flag for the first node of its
-// group (bit 3); and the backward table: per node v, pred(v) with the set of
-// first letters of pred(v)'s group, so that a backward step is one load.
-// select_c uses the line counts plus a sample of the line holding every 64th
+// group (bit 3): a backward step of the prefiltered walk is a select and a
+// scan of at most five nibbles.  select_c uses the line counts plus a sample of the line holding every 64th
 // one.
 #pragma once
 #include "device.cuh"
