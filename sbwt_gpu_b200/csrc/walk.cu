@@ -53,6 +53,10 @@ constexpr u32 kWarps = 4;  // 128-thread blocks
 constexpr u32 kBatch = 32;
 constexpr u32 kPool = 96 + kBatch;
 constexpr u32 kTake = 8;     // idle lanes that take new runs to probe
+// Stretches of at most so many answers are copied by their lanes, all at once; longer ones by the whole warp, one after
+// the other.  In the smallest batches every stretch is one k-mer: 16 reads, 23.5 -> 19.5 us (2, 4 and 8 alike).  Two
+// or four long stretches at a time gave nothing and took registers (10 blocks per SM instead of 12).
+constexpr u32 kOwn = 4;
 constexpr u32 kPiece = 256;  // k-mers per run at most: reads of 250 letters stay whole
 // Batches of fewer k-mers are filled with absent answers by the walk itself: the fill kernel's launch would cost
 // more than it gains.
@@ -186,9 +190,11 @@ __device__ __forceinline__ void set_bits(uint32_t *member, u64 j, u32 count) {
     }
 }
 
-// IX: type of the k-mer and letter indices (u32 where the batch allows it, run32_ok).
+// IX: type of the k-mer and letter indices (u32 where the batch allows it, run32_ok).  12 blocks per SM (40 registers)
+// for u32: 1M own reads, membership only, 323 us against 347 at 10; 14 blocks (36 registers) within 2 % either way.
+// The u64 form would spill there.
 template <class IX>
-__global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker rk, const SearchArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, sizeof(IX) == 4 ? 12 : 10) walk_kernel(const LinesRanker rk, const SearchArgs a) {
     // kernel contract: the run count is on the device; too few runs and the per-k-mer search takes the call
     const u64 n_rows = a.runs_dev ? *a.runs_dev : a.n_rows;
     if (a.runs_dev && !runs_usable(n_rows, a.n_kmers)) return;
@@ -210,6 +216,12 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
         {
             const u32 o_max = k - a.wv.q, qs = 32u - 2u * a.wv.q;
             const u32 two = a.wv.q < 16u ? 1u : 0u;  // 16 letters hold two q-mers
+            // Rounds of a k-mer whose q-mers are present: its right end, its middle, its left end, so that no letter
+            // of it stays unprobed: one substituted letter among the first k - 2 q costs two rounds instead of a failed
+            // look-up for each k-mer that holds it.  Two rounds against three: 10,000 reads, half own, 77 and 65 us;
+            // 230,000 uneven reads 1957 and 1805; 1M own reads, membership only, 323 and 302; four 69, 1845, 323.  In
+            // the smallest batches a run is one k-mer, and a third round only waits (19.5 and 21.5 us for 16 reads).
+            const u32 rounds = a.piece > 1u ? 3u : 2u;
             const IX max_pos = (IX)a.max_pos;
             bool act = false;
             IX pos = 0, J = 0;
@@ -301,9 +313,9 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                 bool pass = false;
                 if (act) {
                     // the letter that ended a stretch is in no indexed k-mer after those before it: the q-mers that
-                    // hold it are probed from the right one on; otherwise the right end, then the middle
+                    // hold it are probed from the right one on; otherwise the right end, the middle and the left end
                     const u32 last = hint ? min(hint - 1u, o_max) : o_max;
-                    const u32 o = hint ? last - 2u * tries : tries ? o_max / 2u : o_max;
+                    const u32 o = hint ? last - 2u * tries : tries == 0u ? o_max : tries == 1u ? o_max / 2u : min(two, o_max);
                     const u32 d = o ? two : 0u;
                     const u32 x = half_words(a, min(pos + (o - d), max_pos), a.wv.q + d);
                     u32 adv = o + 1u;
@@ -314,7 +326,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                     }
                     if (in) {
                         tries++;
-                        pass = tries == 2u || (hint && (o < 2u || o + a.wv.q < hint + 2u));
+                        pass = tries >= (hint ? 3u : rounds) || (hint && (o < 2u || o + a.wv.q < hint + 2u));
                     } else if (adv > left) {
                         act = false;
                     } else {
@@ -392,7 +404,16 @@ __global__ void __launch_bounds__(kWarps * 32, 10) walk_kernel(const LinesRanker
                     if (closed) hint = k;
                 }
                 if (a.answers) {
-                    for (u32 m = __ballot_sync(kFull, count != 0); m; m &= m - 1u) {
+                    if (count && count <= kOwn) {
+                        u32 x[kOwn];
+#pragma unroll
+                        for (u32 t = 0; t < kOwn; t++) x[t] = t < count ? __ldg(a.wv.path_node + at + t) : 0u;
+#pragma unroll
+                        for (u32 t = 0; t < kOwn; t++)
+                            if (t < count) a.answers[J + t] = (u64)x[t];
+                    }
+                    __syncwarp();
+                    for (u32 m = __ballot_sync(kFull, count > kOwn); m; m &= m - 1u) {
                         const int src = __ffs(m) - 1;
                         const u32 c = __shfl_sync(kFull, count, src), f = __shfl_sync(kFull, at, src);
                         u64 *const out = a.answers + __shfl_sync(kFull, J, src);

@@ -80,6 +80,18 @@ def test_walk_batch_sizes(cuda, reads):
         assert np.array_equal(_search(ix, letters, rows, want.size, 1), want)
 
 
+@pytest.mark.parametrize("k", [8, 9, 10, 11, 16, 31])  # 8-letter probes: none to all three offsets fall together
+@pytest.mark.parametrize("reads", [1_000, 5_000])  # runs of one k-mer, and of several
+def test_probes_of_short_and_long_k_mers(cuda, reads, k):
+    rng = wl.rng_for(600 + k)
+    genome = wl.random_bases(rng, 3_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, reads // 2, reads - reads // 2, 150, 0.05)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, 6)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=6) as ix:
+        assert np.array_equal(_search(ix, letters, rows, want.size), want)
+
+
 @pytest.mark.parametrize("rows", [11_263, 11_264])  # the most rows of the one-launch row table, and one more
 @pytest.mark.parametrize("offset", [0, 16, 1])  # alignment of the letters
 def test_row_tables(cuda, rows, offset):
