@@ -403,6 +403,9 @@ __global__ void __launch_bounds__(kWarps * 32, sizeof(IX) == 4 ? 12 : 10) walk_k
                     miss = v == kNoNode || closed;
                     if (closed) hint = k;
                 }
+                // the taken runs are read before other lanes write over their places below; convergence alone (the
+                // ballots) orders no memory
+                __syncwarp();
                 if (a.answers) {
                     if (count && count <= kOwn) {
                         u32 x[kOwn];

@@ -169,3 +169,24 @@ def test_kmer_lists_equal_the_oracle(cuda, k, p):
         l2, r2 = _rows([text[i:i + k] for i in at])
         want2 = orc.OracleIndex(built.bits, built.n_bits).search_reads(l2, r2, k, p)
         assert np.array_equal(pos.cpu().numpy().view(np.uint64), want2)
+
+
+def test_membership_only_with_full_pools(cuda):
+    """Membership alone, with runs that go back to be probed while others are taken from the same pool: reads of
+    which every tenth letter or so is substituted, so that each run changes hands many times."""
+    import torch
+    rng = wl.rng_for(4100)
+    k, p = 21, 8
+    genome = wl.random_bases(rng, 40_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    ox = orc.OracleIndex(built.bits, built.n_bits)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        for length, sub in ((280, 0.01), (280, 0.1), (60, 0.03)):
+            letters, rows = wl.mixed_reads(rng, genome, 20_000, 500, length, sub)
+            want = ox.search_reads(letters, rows, k, p) != orc.NOT_FOUND
+            d_l, d_r = torch.from_numpy(letters).cuda(), torch.from_numpy(rows.view(np.int64)).cuda()
+            for _ in range(3):
+                bits = torch.full(((want.size + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+                ix.search_reads(d_l, d_r, None, want.size, d_member_bits=bits)
+                got = np.unpackbits(bits.cpu().numpy().view(np.uint8), bitorder="little")
+                assert np.array_equal(got[:want.size].astype(bool), want) and not got[want.size:].any()
