@@ -83,8 +83,9 @@ struct Train {
             at += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
         }
     };
-    // own_batch: room for the batch's k-mers and labels as well.
-    int setup(uint32_t batch, uint32_t kk, uint32_t hist, bool own_batch = false) {
+    // own_batch: room for the batch's k-mers and labels as well.  s: the stream that trains; the state is cleared on
+    // it (cudaMemset would clear on the legacy stream, which a non-blocking stream does not wait for).
+    int setup(uint32_t batch, uint32_t kk, uint32_t hist, cudaStream_t s, bool own_batch = false) {
         B = batch;
         k = kk;
         const uint32_t P = off.count;
@@ -120,7 +121,7 @@ struct Train {
         }
         loss_sum = grad + P;
         if (own_batch) kmers = km, labels = lb, n_train = B;
-        SBWT_CHECK_CUDA(cudaMemset(arena, 0, zeroed));
+        SBWT_CHECK_CUDA(cudaMemsetAsync(arena, 0, zeroed, s));
         return 0;
     }
     // the BF16 operand copies of W1, W2 and W2's transpose from theta
@@ -309,7 +310,7 @@ extern "C" int sbwt_prefilter_train(sbwt_index *ix, const sbwt_mlp_params *prm, 
         t.kmers = d_train;
         t.labels = d_labels;
         const uint32_t hist_every = 100;
-        if ((rc = t.setup(prm->batch, ix->k, prm->steps / hist_every + 1)) != 0) break;
+        if ((rc = t.setup(prm->batch, ix->k, prm->steps / hist_every + 1, s)) != 0) break;
         const std::vector<float> th0 = init_theta(t.off, ix->k, prm->seed ^ 0xA5A5A5A5ull);
         SBWT_CHECK_CUDA(cudaMemcpyAsync(t.theta, th0.data(), th0.size() * sizeof(float), cudaMemcpyHostToDevice, s));
         if ((rc = t.refresh_bf16(s)) != 0) break;
@@ -598,7 +599,7 @@ extern "C" int sbwt_mlp_gradients(uint32_t k, const float *theta, const uint64_t
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return set_error("no CUDA device is available");
     Train t;
-    SBWT_TRY(t.setup(n, k, 1, true));
+    SBWT_TRY(t.setup(n, k, 1, 0, true));
     uint64_t *d_k = const_cast<uint64_t *>(t.kmers);
     uint8_t *d_l = const_cast<uint8_t *>(t.labels);
     SBWT_CHECK_CUDA(cudaMemcpy(d_k, kmers, (size_t)n * 8, cudaMemcpyHostToDevice));

@@ -256,3 +256,25 @@ def test_sandwich_holds_when_the_index_has_more_kmers_than_the_training_set(cuda
             assert st["n_rejected_indexed"] == st["n_indexed_kmers"] > 250_000
             skipped, nk, want = _filtered_vs_oracle(ix, pf, built, letters, rows, k, 10, cuda)
     assert (want != orc.NOT_FOUND).any() and 0 < skipped < nk
+
+
+def test_training_state_is_cleared_before_it_is_used(trained, cuda):
+    """Training on a stream of its own while the default stream is busy: the step counter, the moments and the loss
+    history are cleared in the order of the training, not behind what the default stream still has to do.  Three
+    steps move a parameter by at most 3 lr (Adam with its bias corrections; equal gradients may differ in the order of
+    their sums and so in the sign of a step where they vanish), and the first loss depends on no such order but the
+    sum's own (8,192 terms in FP32)."""
+    import torch
+    kw = dict(steps=3, batch=8192, lr=1e-3, n_positive=8192, n_negative=8192, seed=11)
+    runs = []
+    a = torch.randn(8192, 8192, device=cuda, dtype=torch.bfloat16)
+    for busy in (False, True):
+        torch.cuda.synchronize()
+        for _ in range(400 if busy else 0):  # about 0.3 s
+            torch.matmul(a, a)
+        with sg.Prefilter.train(trained["ix"], **kw) as pf:
+            runs.append((pf.stats(), pf.params()))
+    torch.cuda.synchronize()
+    (s0, p0), (s1, p1) = runs
+    assert abs(s0["first_loss"] - s1["first_loss"]) < 1e-4 and 0.3 < s0["first_loss"] < 1.5
+    assert np.isfinite(p1).all() and np.abs(p0 - p1).max() <= 2 * 3 * 1.01e-3
