@@ -596,11 +596,13 @@ int search_rows_device(sbwt_index *ix, Workspace &w, const uint8_t *d_letters, u
     bool capturing = false;
     if (ix->use_graph && !prof && s != nullptr) {
         const KernelShape &sh = ix->shape;
-        const uint64_t key[12] = {(uint64_t)d_letters, n_letters, (uint64_t)d_rows, n_rows, (uint64_t)d_answers,
-                                  (uint64_t)d_member, n_kmers, (uint64_t)s, ix->gen,
-                                  ((uint64_t)sh.layout << 48) | ((uint64_t)sh.mode << 40) | ((uint64_t)sh.kpt << 32) |
-                                      ((uint64_t)sh.tpk << 16) | sh.tpb,
-                                  (uint64_t)w.words ^ (uint64_t)w.kstart, (uint64_t)w.chunk_row ^ (uint64_t)w.counter};
+        // every pointer the captured launches hold: scan too, which sbwt_search_packed grows on its own
+        const uint64_t key[Workspace::kGraphKey] = {
+            (uint64_t)d_letters, n_letters, (uint64_t)d_rows, n_rows, (uint64_t)d_answers, (uint64_t)d_member, n_kmers,
+            (uint64_t)s, ix->gen,
+            ((uint64_t)sh.layout << 48) | ((uint64_t)sh.mode << 40) | ((uint64_t)sh.kpt << 32) |
+                ((uint64_t)sh.tpk << 16) | sh.tpb,
+            (uint64_t)w.words, (uint64_t)w.kstart, (uint64_t)w.chunk_row, (uint64_t)w.counter, (uint64_t)w.scan};
         if (w.graph && std::memcmp(key, w.graph_key, sizeof key) == 0) {
             SBWT_CHECK_CUDA(cudaGraphLaunch(w.graph, s));
             return 0;

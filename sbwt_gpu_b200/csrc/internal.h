@@ -113,7 +113,8 @@ struct Workspace {
     // CUDA graph of the last pack -> table -> search -> bitmap chain, replayed
     // while every launch parameter (the key) stays the same
     cudaGraphExec_t graph = nullptr;
-    uint64_t graph_key[12] = {0};
+    static constexpr int kGraphKey = 15;
+    uint64_t graph_key[kGraphKey] = {0};
     void release();
 };
 

@@ -190,3 +190,34 @@ def test_membership_only_with_full_pools(cuda):
                 ix.search_reads(d_l, d_r, None, want.size, d_member_bits=bits)
                 got = np.unpackbits(bits.cpu().numpy().view(np.uint8), bitorder="little")
                 assert np.array_equal(got[:want.size].astype(bool), want) and not got[want.size:].any()
+
+
+def test_graph_replay_after_the_kernel_contract(cuda):
+    """The kernel contract grows scratch that a captured search of reads uses: the next search captures again."""
+    import torch
+    rng = wl.rng_for(4200)
+    k, p = 31, 10
+    genome = wl.random_bases(rng, 40_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, 6_000, 6_000, 60, 0.01)  # more rows than one launch prepares
+    ox = orc.OracleIndex(built.bits, built.n_bits)
+    want = ox.search_reads(letters, rows, k, p)
+    words = torch.from_numpy(wl.pack_words(genome).view(np.int64)).cuda()
+    s = torch.cuda.Stream()
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        ix.use_graphs(True)
+        d_l, d_r = torch.from_numpy(letters).cuda(), torch.from_numpy(rows.view(np.int64)).cuda()
+        ans = torch.empty(want.size, dtype=torch.int64, device="cuda")
+        for contract in (0, 30_000, 39_000):
+            if contract:
+                pos = torch.arange(contract, dtype=torch.int64, device="cuda")
+                torch.cuda.synchronize()
+                ix.search_packed(words, pos, stream=s)
+                s.synchronize()
+                ref = ox.search_reads(genome[:contract + k - 1], np.array([0, contract + k - 1], dtype=np.uint64), k, p)
+                assert np.array_equal(pos.cpu().numpy().view(np.uint64), ref)
+            ans.fill_(-7)
+            torch.cuda.synchronize()
+            ix.search_reads(d_l, d_r, ans, want.size, stream=s)
+            s.synchronize()
+            assert np.array_equal(ans.cpu().numpy().view(np.uint64), want)
