@@ -83,9 +83,15 @@ extern "C" int sbwt_search_reads_noalloc(sbwt_index *ix, const uint8_t *d_letter
     const size_t off_kstart = 256;
     const size_t off_scan = align256(off_kstart + (n_rows + 1) * sizeof(u64));
     const size_t off_chunks = align256(off_scan + scan_scratch_words(n_rows) * sizeof(u64));
-    const size_t off_words = align256(off_chunks + ((n_kmers + a.chunk - 1) / a.chunk) * sizeof(u32));
-    const size_t off_answers = align256(off_words + n_words * sizeof(u64));
-    const size_t need = scratch_answers ? off_answers + n_kmers * sizeof(u64) : off_words + n_words * sizeof(u64);
+    size_t off_words = 0, off_answers = 0, need = 0;
+    for (;;) {
+        off_words = align256(off_chunks + ((n_kmers + a.chunk - 1) / a.chunk) * sizeof(u32));
+        off_answers = align256(off_words + n_words * sizeof(u64));
+        need = scratch_answers ? off_answers + n_kmers * sizeof(u64) : off_words + n_words * sizeof(u64);
+        // the walk's smallest chunks only where their table fits: none takes more room than one of whole windows
+        if (need <= kNoAllocBytes || !a.walk || a.chunk >= search_chunk(ix, true)) break;
+        a.chunk *= 2u;
+    }
     if (need > kNoAllocBytes)
         return set_error("sbwt_search_reads_noalloc: this batch (%llu letters, %llu rows, %llu k-mers) needs %zu "
                          "bytes of scratch, more than the fixed %zu; split the batch or use sbwt_search_reads",

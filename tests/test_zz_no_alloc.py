@@ -83,3 +83,37 @@ def test_noalloc_rejects_a_batch_beyond_its_scratch(cuda):
         assert b"scratch" in err and b"bytes" in err
         assert _noalloc(ix, d_l, d_r, None, n_letters - 30) != 0  # NULL answers and no bitmap
         assert b"NULL" in _lib.lib.sbwt_last_error()
+
+
+def test_noalloc_takes_a_small_batch_of_many_rows_up_to_its_scratch(cuda):
+    """A batch whose row table all but fills the scratch, with few k-mers: the chunk table of a small batch, which has
+    shorter chunks, must not be what refuses it."""
+    import torch
+    rng = wl.rng_for(608)
+    k = 31
+    genome = wl.random_bases(rng, 50_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, 400, 400, 150, 0.01)
+    nk = sg.count_kmers(rows, k)
+
+    def need(n_rows):  # bytes, with a chunk of 128 k-mers: counter | row table | scan | chunk table | words
+        at = 256
+        for size in ((n_rows + 1) * 8, ((n_rows + 1023) // 1024 + 2) * 8, (nk + 127) // 128 * 4):
+            at = (at + size + 255) // 256 * 256
+        return at + (letters.size + 63) // 32 * 8
+
+    n_rows = (32 << 20) // 8
+    while need(n_rows) > 32 << 20:
+        n_rows -= 1
+    d_r = torch.full((n_rows + 1,), letters.size, dtype=torch.int64, device=cuda)  # the other rows are empty
+    d_r[: rows.size] = torch.from_numpy(rows.view(np.int64)).to(cuda)
+    d_l = torch.from_numpy(letters).to(cuda)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, 8)
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=8) as ix:
+        got = torch.full((nk,), -3, dtype=torch.int64, device=cuda)
+        assert _noalloc(ix, d_l, d_r, got, nk) == 0, _lib.lib.sbwt_last_error()
+        torch.cuda.synchronize()
+        assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+        more = torch.cat([d_r, d_r[-1:].expand(64)])
+        assert _noalloc(ix, d_l, more, got, nk) != 0  # past the scratch whatever the chunks
+        assert b"scratch" in _lib.lib.sbwt_last_error()
