@@ -343,10 +343,14 @@ uint64_t sbwt_count_kmers(const uint64_t *row_starts, uint64_t n_rows, uint32_t 
  * 32-byte lines and the 512/2048-bit wide lines, with SBWT_TUNE_POPPY also
  * the poppy layouts SB 512/1024/2048, with SBWT_TUNE_SHAPES also the
  * per-k-mer kernel's shapes (k-mers per thread {1,2,3,4,6,8} x threads per
- * k-mer {1,2,4} x threads per block {128,256}); (2) the run walk's knobs on
+ * k-mer {1,2,4} x threads per block {128,256}); (2) the walk's knobs on
  * the best layout (window 64/128/256 k-mers, resident blocks per SM, the
- * evict-first policy of the table gathers, compact presearch entries); (3)
- * with SBWT_TUNE_P the presearch depth {8,10,12,14,15} <= k.  Checks that
+ * evict-first policy of the presearch gathers, the L2 set-aside, and with
+ * SBWT_SEARCH_SKIP_ABSENT compact presearch entries); (3) with SBWT_TUNE_P
+ * the presearch depth {8,10,12,14,15} <= k.  The index's search mode stays.
+ * With SBWT_SEARCH_STREAM the walk reads the 32-byte lines whatever the
+ * layout, so those are the layout it leaves, and the other layouts are timed
+ * with SBWT_SEARCH_SKIP_ABSENT, for the report and the check.  Checks that
  * every candidate's answers have the same checksum, and leaves the fastest
  * configured on the index.  d_answers: device scratch of n_kmers u64.
  * report (optional): JSON of the choice, the time of the configuration

@@ -11,12 +11,16 @@
 //      reference's poppy layouts (SB 512/1024/2048), with SBWT_TUNE_SHAPES
 //      also the per-k-mer kernel's register shapes (k-mers per thread
 //      {1,2,3,4,6,8} x threads per k-mer {1,2,4} x threads per block
-//      {128,256});
-//   2. the run walk's knobs on the best layout, one at a time, each kept
+//      {128,256}).  The forward walk reads the 32-byte lines whatever the
+//      layout: where the index's mode takes it, the lines are the only layout
+//      it can choose, and the others are timed (and their answers checked)
+//      with the absent-run skip, which does rank in them;
+//   2. the walk's knobs on the best layout, one at a time, each kept
 //      when it is faster: window (64 / 256 k-mers against 128), resident
 //      blocks per SM, the evict-first policy of the presearch gathers
-//      (never / always against by table size), the rank lines held in the persisting L2 set-aside, and the compact
-//      4-byte presearch entries;
+//      (never / always against by table size), the rank lines held in the
+//      persisting L2 set-aside, and, where the right-to-left walk is taken, the
+//      compact 4-byte presearch entries (the forward walk does not read them);
 //   3. with SBWT_TUNE_P the presearch depth p in {8,10,12,14,15} (p <= k),
 //      then the window and the evict policy again at the chosen p.
 // Every candidate's answers are reduced to an order-sensitive checksum, and
@@ -49,8 +53,10 @@ struct Cand {
     u32 p;
     u32 window, bps;
     int evict, compact, persist;
+    int mode;
     float ms;
     unsigned long long sum;
+    bool walk;  // measured with the forward walk
 };
 
 const char *layout_name(int l) {
@@ -58,14 +64,19 @@ const char *layout_name(int l) {
                                                                                                           : "lines2048";
 }
 
+const char *mode_name(int m) {
+    return m == SBWT_SEARCH_STREAM ? "stream" : m == SBWT_SEARCH_SKIP_ABSENT ? "skip" : "every";
+}
+
 std::string cand_json(const Cand &c) {
     char b[384];
     std::snprintf(b, sizeof b,
-                  "{\"layout\":\"%s\",\"kmers_per_thread\":%u,\"threads_per_kmer\":%u,\"threads_per_block\":%u,"
+                  "{\"layout\":\"%s\",\"mode\":\"%s\",\"kmers_per_thread\":%u,\"threads_per_kmer\":%u,"
+                  "\"threads_per_block\":%u,"
                   "\"bits_in_superblock\":%u,\"shuffles\":%d,\"p\":%u,\"window\":%u,\"blocks_per_sm\":%u,"
                   "\"evict\":\"%s\",\"compact_presearch\":%d,\"l2_persist\":%d,\"ms\":%.4f}",
-                  layout_name(c.layout), c.kpt, c.tpk, c.tpb, c.sb, c.shuffles, c.p, c.window, c.bps,
-                  c.evict == 0 ? "by table size" : c.evict == 1 ? "never" : "always", c.compact, c.persist, c.ms);
+                  layout_name(c.layout), mode_name(c.mode), c.kpt, c.tpk, c.tpb, c.sb, c.shuffles, c.p, c.window,
+                  c.bps, c.evict == 0 ? "by table size" : c.evict == 1 ? "never" : "always", c.compact, c.persist, c.ms);
     return b;
 }
 
@@ -113,6 +124,7 @@ extern "C" int sbwt_autotune(sbwt_index *ix, const uint8_t *d_letters, uint64_t 
         ix->shape.blocks_per_sm = c.bps;
         ix->shape.evict = c.evict;
         ix->shape.l2_persist = c.persist;
+        ix->shape.mode = c.mode;
         if (!c.persist && ix->l2_setaside) l2_setaside_release(ix);  // a set-aside without the window costs L2
         if (c.p != ix->p || c.compact != ix->compact_pre) {
             ix->compact_pre = c.compact;
@@ -123,6 +135,7 @@ extern "C" int sbwt_autotune(sbwt_index *ix, const uint8_t *d_letters, uint64_t 
     };
     auto measure = [&](Cand &c) -> int {
         SBWT_TRY(apply(c));
+        c.walk = stream_form(ix);
         Workspace &w = ix->ws[0];
         SBWT_TRY(search_rows_device(ix, w, d_letters, n_letters, d_row_starts, n_rows, d_answers, nullptr, n_kmers, s));
         float best = 1e30f;
@@ -162,17 +175,21 @@ extern "C" int sbwt_autotune(sbwt_index *ix, const uint8_t *d_letters, uint64_t 
         const int c0 = ix->compact_pre;
         // stage 1: layouts; the first candidate is the index's configuration before tuning
         std::vector<Cand> stage1;
+        const int mode = saved.mode;
+        // the mode of the queue-fed layouts beside the lines
+        const int other = mode == SBWT_SEARCH_STREAM && ix->stream_ok && ix->walk_q ? SBWT_SEARCH_SKIP_ABSENT : mode;
         stage1.push_back(Cand{saved.layout, saved.kpt, saved.tpk, saved.tpb, saved.sb, saved.shuffles, p0,
-                              saved.window, saved.blocks_per_sm, saved.evict, c0, saved.l2_persist, 0, 0});
+                              saved.window, saved.blocks_per_sm, saved.evict, c0, saved.l2_persist, mode});
         if (ix->lines_ok) {
             for (int l : {SBWT_LAYOUT_LINES, SBWT_LAYOUT_LINES512, SBWT_LAYOUT_LINES2048})
                 if (!(l == saved.layout && saved.kpt == 0 && saved.tpk == 1))
-                    stage1.push_back(Cand{l, 0, 1, 128, 1024, 0, p0, 128, 0, 0, c0, 0, 0, 0});
+                    stage1.push_back(Cand{l, 0, 1, 128, 1024, 0, p0, 128, 0, 0, c0, 0,
+                                          l == SBWT_LAYOUT_LINES ? mode : other});
             if (flags & 8u)
                 for (u32 tpb : {128u, 256u})
                     for (u32 tpk : {1u, 2u, 4u})
                         for (u32 kpt : {1u, 2u, 3u, 4u, 6u, 8u})
-                            stage1.push_back(Cand{SBWT_LAYOUT_LINES, kpt, tpk, tpb, 1024, 0, p0, 128, 0, 0, c0, 0, 0, 0});
+                            stage1.push_back(Cand{SBWT_LAYOUT_LINES, kpt, tpk, tpb, 1024, 0, p0, 128, 0, 0, c0, 0, mode});
         }
         if ((flags & 4u) || !ix->lines_ok)
             for (u32 sb : {512u, 1024u, 2048u})
@@ -182,15 +199,20 @@ extern "C" int sbwt_autotune(sbwt_index *ix, const uint8_t *d_letters, uint64_t 
                         if (kpt == 0 && sh) continue;
                         if (kpt && !(flags & 8u)) continue;
                         stage1.push_back(Cand{SBWT_LAYOUT_POPPY, kpt, 1, kpt == 0 ? 128u : 256u, sb, sh, p0, 128, 0, 0,
-                                              c0, 0, 0, 0});
+                                              c0, 0, kpt == 0 ? other : mode});
                     }
                 }
         for (Cand &c : stage1)
             if ((rc = measure(c)) != 0) break;
         if (rc) break;
         default_ms = done.front().ms;
-        Cand best = *std::min_element(done.begin(), done.end(), [](const Cand &a, const Cand &b) { return a.ms < b.ms; });
-        // stage 2: the run walk's knobs, one at a time (kept when faster by more than 1 %)
+        // the index's mode stays; a walk is one and the same on every layout, and the reads behind the prefilter
+        // need the lines
+        auto eligible = [&](const Cand &c) { return c.mode == mode && (!c.walk || c.layout == SBWT_LAYOUT_LINES); };
+        Cand best = *std::min_element(done.begin(), done.end(), [&](const Cand &a, const Cand &b) {
+            return eligible(a) != eligible(b) ? eligible(a) : a.ms < b.ms;
+        });
+        // stage 2: the walk's knobs, one at a time (kept when faster by more than 1 %)
         auto try_knob = [&](Cand c) -> int {
             SBWT_TRY(measure(c));
             if (c.ms < 0.99f * best.ms) best = c;
@@ -220,7 +242,7 @@ extern "C" int sbwt_autotune(sbwt_index *ix, const uint8_t *d_letters, uint64_t 
                 c.persist = best.persist ? 0 : 1;
                 SBWT_TRY(try_knob(c));
             }
-            if (compact && ix->n < dev::kPreMaxColumns && best.p) {
+            if (compact && !best.walk && ix->n < dev::kPreMaxColumns && best.p) {
                 Cand c = best;
                 c.compact = best.compact == 1 ? 0 : 1;
                 SBWT_TRY(try_knob(c));

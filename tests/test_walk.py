@@ -221,3 +221,37 @@ def test_graph_replay_after_the_kernel_contract(cuda):
             ix.search_reads(d_l, d_r, ans, want.size, stream=s)
             s.synchronize()
             assert np.array_equal(ans.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("layout", [sg.SBWT_LAYOUT_LINES, sg.SBWT_LAYOUT_POPPY])
+def test_autotune_tries_what_the_walk_reads(cuda, layout):
+    """The forward walk is the same on every layout: the tuner leaves the lines, times the others with kernels that
+    read them, tries no table that the walk does not read, and the reads behind the prefilter still run."""
+    import torch
+    rng = wl.rng_for(4300)
+    k, p = 31, 8
+    genome = wl.random_bases(rng, 30_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, 200, 200, 150, 0.01)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, p)
+    d_l, d_r = torch.from_numpy(letters).cuda(), torch.from_numpy(rows.view(np.int64)).cuda()
+    ans = torch.empty(want.size, dtype=torch.int64, device="cuda")
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        ix.configure(layout)
+        rep = ix.autotune(d_l, d_r, ans, want.size, tune_poppy=True)
+        cands = rep["candidates"]
+        assert rep["best"]["layout"] == "lines" and rep["best"]["mode"] == "stream"
+        assert {c["layout"] for c in cands if c["mode"] == "skip"} == {"lines512", "lines2048", "poppy"}
+        assert all(c["layout"] == "lines" for c in cands[1:] if c["mode"] == "stream")
+        assert len({c["compact_presearch"] for c in cands}) == 1
+        with sg.Prefilter.train(ix, steps=20, batch=256, n_positive=2_000, n_negative=2_000) as pf:
+            ans.fill_(-7)
+            ix.search_reads_filtered(pf, d_l, d_r, ans, want.size)
+            torch.cuda.synchronize()
+            assert np.array_equal(ans.cpu().numpy().view(np.uint64), want)
+        ix.set_search_mode(sg.SEARCH_SKIP_ABSENT)  # the layouts differ: any may be left
+        rep = ix.autotune(d_l, d_r, ans, want.size, tune_poppy=True)
+        assert {c["mode"] for c in rep["candidates"]} == {"skip"}
+        assert len({c["compact_presearch"] for c in rep["candidates"]}) == 2
+        torch.cuda.synchronize()
+        assert np.array_equal(ans.cpu().numpy().view(np.uint64), want)
