@@ -465,12 +465,13 @@ namespace sbwt {
 
 // Option (KernelShape.l2_persist, environment SBWT_L2_PERSIST=1, tried by
 // the autotuner): the search launch carries an access-policy window over the
-// current layout's rank lines with the persisting property, and the index
+// rank lines that it reads (the current layout's; the forward walk the 32-byte
+// lines on every layout) with the persisting property, and the index
 // sizes the device's persisting L2 set-aside to hold them (a CUDA context
 // limit, taken on the first such launch and released when the last index
 // that took it is freed).  Layouts larger than the set-aside (poppy, or lines
-// beyond it) get no window.  Measured on the large workload: 8.64 ms a
-// launch against 8.33 ms without (the lines are not what misses L2; the L2
+// beyond it) get no window.  Measured on the large workload with the
+// right-to-left walk: 8.64 ms a launch against 8.33 ms without (the lines are not what misses L2; the L2
 // hit rate stays at 20 %), and 11.4 ms with the set-aside carved out of L2
 // but no window, so it is off by default.
 namespace {
@@ -480,13 +481,13 @@ int g_l2_users[kL2Devices] = {0};   // live indexes holding the set-aside
 size_t g_l2_set[kL2Devices] = {0};  // its size: the largest any of them asked for
 }  // namespace
 
-bool l2_window(const sbwt_index *ix, cudaAccessPolicyWindow *w) {
+bool l2_window(const sbwt_index *ix, bool walk, cudaAccessPolicyWindow *w) {
     if (!ix->shape.l2_persist) return false;
     if (ix->l2_setaside == 0) l2_setaside_acquire(const_cast<sbwt_index *>(ix));  // first windowed launch
     if (ix->l2_setaside == 0) return false;
     const void *base = nullptr;
     size_t bytes = 0;
-    if (ix->shape.layout == SBWT_LAYOUT_LINES && ix->lines_ok) {
+    if ((walk || ix->shape.layout == SBWT_LAYOUT_LINES) && ix->lines_ok) {
         base = ix->d_lines, bytes = 4ull * ix->lpc * sizeof(ulonglong4);
     } else if (wide_sectors(ix->shape.layout) && ix->wide_s == wide_sectors(ix->shape.layout)) {
         base = ix->d_wide, bytes = 4ull * ix->wide_lpc * ix->wide_s * sizeof(ulonglong4);

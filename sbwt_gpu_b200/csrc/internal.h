@@ -252,10 +252,10 @@ int search_rows_device(sbwt_index *ix, Workspace &w, const uint8_t *d_letters, u
 template <class T> int grow(T *&p, size_t &cap, size_t need);
 template <class T> int grow_host(T *&p, size_t &cap, size_t need);
 
-// api.cu: the L2 access-policy window of a search launch over the index's
-// current layout (false: none applies); l2_setaside_acquire/release size the
+// api.cu: the L2 access-policy window of a search launch over the rank lines of
+// the index's current layout, or of the forward walk (false: none applies); l2_setaside_acquire/release size the
 // device's persisting set-aside for the indexes that use it.
-bool l2_window(const sbwt_index *ix, cudaAccessPolicyWindow *w);
+bool l2_window(const sbwt_index *ix, bool walk, cudaAccessPolicyWindow *w);
 int l2_setaside_acquire(sbwt_index *ix);
 void l2_setaside_release(sbwt_index *ix);
 

@@ -16,7 +16,7 @@ int launch_kernel(K kern, u32 blocks, u32 threads, cudaStream_t s, const sbwt_in
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.numAttrs = 0;
-    if (l2_window(ix, &attr[0].val.accessPolicyWindow)) {
+    if (l2_window(ix, a.walk, &attr[0].val.accessPolicyWindow)) {
         attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
         cfg.attrs = attr;
         cfg.numAttrs = 1;

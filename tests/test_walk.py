@@ -255,3 +255,39 @@ def test_autotune_tries_what_the_walk_reads(cuda, layout):
         assert len({c["compact_presearch"] for c in rep["candidates"]}) == 2
         torch.cuda.synchronize()
         assert np.array_equal(ans.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("layout", [sg.SBWT_LAYOUT_LINES, sg.SBWT_LAYOUT_LINES512, sg.SBWT_LAYOUT_POPPY])
+def test_the_l2_window_covers_the_lines_that_the_walk_reads(cuda, layout):
+    import torch
+    from cuda.bindings import runtime as rt
+    rng = wl.rng_for(4400)
+    k, p = 31, 8
+    genome = wl.random_bases(rng, 30_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, 50, 50, 150, 0.01)
+    nk = sg.count_kmers(rows, k)
+    d_l, d_r = torch.from_numpy(letters).cuda(), torch.from_numpy(rows.view(np.int64)).cuda()
+    ans = torch.empty(nk, dtype=torch.int64, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        ix.configure(layout)
+        ix.set_walk_options(l2_persist=1)
+        ix.search_reads(d_l, d_r, ans, nk, stream=s)  # takes the set-aside and the workspace
+        s.synchronize()
+        assert rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)[0] == 0
+        ix.search_reads(d_l, d_r, ans, nk, stream=s)
+        err, graph = rt.cudaStreamEndCapture(s.cuda_stream)
+        assert err == 0
+        count = rt.cudaGraphGetNodes(graph)[-1]
+        windows = []
+        for node in rt.cudaGraphGetNodes(graph, count)[1]:
+            if rt.cudaGraphNodeGetType(node)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel:
+                err, val = rt.cudaGraphKernelNodeGetAttribute(
+                    node, rt.cudaLaunchAttributeID.cudaLaunchAttributeAccessPolicyWindow)
+                assert err == 0
+                windows.append(int(val.accessPolicyWindow.num_bytes))
+        rt.cudaGraphDestroy(graph)
+    lines = (built.n_bits // 224 + 1 + 7) // 8 * 8
+    assert max(windows) == 4 * lines * 32
