@@ -291,3 +291,32 @@ def test_the_l2_window_covers_the_lines_that_the_walk_reads(cuda, layout):
         rt.cudaGraphDestroy(graph)
     lines = (built.n_bits // 224 + 1 + 7) // 8 * 8
     assert max(windows) == 4 * lines * 32
+
+
+@pytest.mark.parametrize("order", ["reads", "shuffled"])
+def test_kernel_contract_of_a_batch_that_is_filled_ahead(cuda, order):
+    """From 8M k-mers on the absent answers are written before the walk, over the caller's positions: only where the
+    walk takes the call.  Shuffled, the positions form no runs and the list search still has to find them there.  The
+    answers start off the 32-byte stores' alignment."""
+    import torch
+    rng = wl.rng_for(4500)
+    k, p, reads, length = 31, 10, 71_000, 149
+    genome = wl.random_bases(rng, 50_000)
+    built = sg.build_sbwt([genome.tobytes()], k)
+    letters, rows = wl.mixed_reads(rng, genome, reads // 4, reads - reads // 4, length, 0.01)
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, p)
+    assert want.size > 8 << 20
+    per = length - k + 1
+    pos = (np.arange(reads, dtype=np.int64)[:, None] * length + np.arange(per)).reshape(-1)
+    if order == "shuffled":
+        at = rng.permutation(pos.size)
+        pos, want = pos[at], want[at]
+    words = torch.from_numpy(wl.pack_words(letters).view(np.int64)).cuda()
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=p) as ix:
+        buf = torch.full((pos.size + 4,), -7, dtype=torch.int64, device="cuda")
+        buf[1:1 + pos.size] = torch.from_numpy(pos).cuda()
+        ix.search_packed(words, buf[1:1 + pos.size], pos.size)
+        torch.cuda.synchronize()
+        got = buf.cpu().numpy().view(np.uint64)
+        assert np.array_equal(got[1:1 + pos.size], want)
+        assert (got[:1] == np.uint64(2**64 - 7)).all() and (got[1 + pos.size:] == np.uint64(2**64 - 7)).all()
