@@ -302,7 +302,10 @@ __global__ void keys_kernel(u32 n, u32 n_pad, u32 k, u64 *__restrict__ code, con
 
 // What the forward walk relies on, for every column: keys ascend, strictly
 // between labels without $; only group starts have outgoing edges; a group has
-// at most 5 members.  An index whose k is not the one it was built for fails.
+// at most 5 members.  With a smaller k than the index's this fails where two
+// labels agree in their last k letters.  Where none do, and with a larger k,
+// labels, groups and edges stay consistent (a label is what the edges spell
+// backwards, as in the search), and the forward walk serves that k.
 __global__ void walk_check_kernel(u32 n, u32 k, const u64 *__restrict__ keys, const uint8_t *__restrict__ node,
                                   const u32 *__restrict__ marks, const ulonglong4 *__restrict__ lines, u32 lpc,
                                   unsigned long long *__restrict__ bad) {

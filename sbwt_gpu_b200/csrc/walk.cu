@@ -4,12 +4,13 @@
 // (include/gpu/search_kernel.hpp:61-104); no reference counterpart.
 //
 // What is known of a run decides how its next k-mers are found:
-//  * probe: a k-mer with a q-mer (q = 11..16 letters) that no indexed k-mer
-//    contains is absent, and so is every other k-mer that contains that q-mer.
-//    One bit per possible q-mer (WalkView.qbits, L2-resident) tells.  The q-mers
-//    are probed from the right end of the k-mer, so that an absent one at offset
-//    o settles the o + 1 k-mers from the current one on; random letters are
-//    settled k-q+1 k-mers at a time with no access to the index proper.
+//  * probe: a k-mer with a q-mer (q letters, by the index's size: walk_q, 16
+//    and k at most) that no indexed k-mer contains is absent, and so is every
+//    other k-mer that contains that q-mer.  One bit per possible q-mer
+//    (WalkView.qbits, L2-resident) tells.  The q-mers are probed from the right
+//    end of the k-mer, so that an absent one at offset o settles the o + 1
+//    k-mers from the current one on; random letters are settled k-q+1 k-mers at
+//    a time with no access to the index proper.
 //  * lookup, when the probed q-mers are all present: the nodes whose labels end
 //    with the k-mer's last p letters are the presearch interval of those
 //    letters, and labels are sorted, so a search by halves over the keys of
@@ -54,7 +55,7 @@ constexpr u32 kBatch = 32;
 constexpr u32 kPool = 96 + kBatch;
 constexpr u32 kTake = 8;     // idle lanes that take new runs to probe
 // Stretches of at most so many answers are copied by their lanes, all at once; longer ones by the whole warp, one after
-// the other.  In the smallest batches every stretch is one k-mer: 16 reads, 23.5 -> 19.5 us (2, 4 and 8 alike).  Two
+// the other.  In the smallest batches every stretch is one k-mer: 16 reads, 18.4 -> 13.5 us (2, 4 and 8 alike).  Two
 // or four long stretches at a time gave nothing and took registers (10 blocks per SM instead of 12).
 constexpr u32 kOwn = 4;
 constexpr u32 kPiece = 256;  // k-mers per run at most: reads of 250 letters stay whole
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kWarps * 32, sizeof(IX) == 4 ? 12 : 10) walk_k
             // of it stays unprobed: one substituted letter among the first k - 2 q costs two rounds instead of a failed
             // look-up for each k-mer that holds it.  Two rounds against three: 10,000 reads, half own, 77 and 65 us;
             // 230,000 uneven reads 1957 and 1805; 1M own reads, membership only, 323 and 302; four 69, 1845, 323.  In
-            // the smallest batches a run is one k-mer, and a third round only waits (19.5 and 21.5 us for 16 reads).
+            // the smallest batches a run is one k-mer, and a third round only waits (13.0 and 14.3 us for 16 reads).
             const u32 rounds = a.piece > 1u ? 3u : 2u;
             const IX max_pos = (IX)a.max_pos;
             bool act = false;

@@ -320,3 +320,35 @@ def test_kernel_contract_of_a_batch_that_is_filled_ahead(cuda, order):
         got = buf.cpu().numpy().view(np.uint64)
         assert np.array_equal(got[1:1 + pos.size], want)
         assert (got[:1] == np.uint64(2**64 - 7)).all() and (got[1 + pos.size:] == np.uint64(2**64 - 7)).all()
+
+
+@pytest.mark.parametrize("kind,dk,walks", [("plain", -2, True), ("plain", 1, True), ("variants", -2, False),
+                                           ("variants", -1, False), ("variants", 1, True), ("variants", 3, True)])
+def test_which_walk_another_k_takes(cuda, kind, dk, walks):
+    """A smaller k than the index's makes labels equal where sequences differ only in the letters that it drops: the
+    check of the structures finds them and the right-to-left walk searches.  A larger one, or a smaller one that makes
+    none equal, leaves the structures consistent, and the forward walk searches, with the same answers.  (A small
+    batch takes a few blocks of the forward walk; the other one's grid fills the device.)"""
+    import torch
+    rng = wl.rng_for(4600)
+    k = 21 + dk
+    genome = wl.random_bases(rng, 8_000)
+    seqs = [genome.tobytes()]
+    if kind == "variants":
+        for _ in range(3):
+            var = genome.copy()
+            wl.substitute(rng, var, 0.02)
+            seqs.append(var.tobytes())
+    built = sg.build_sbwt(seqs, 21)
+    parts = [s[at:at + 90].decode() for s in seqs for at in rng.integers(0, 7_900, size=24 // len(seqs))]
+    letters, rows = _rows(parts + [wl.random_bases(rng, 90).tobytes().decode() for _ in range(4)])
+    want = orc.OracleIndex(built.bits, built.n_bits).search_reads(letters, rows, k, 8)
+    assert 0.3 < (want != orc.NOT_FOUND).mean() < 0.95
+    with sg.Index.from_bits(built.bits, built.n_bits, k=k, k_presearch=8) as ix:
+        assert np.array_equal(_search(ix, letters, rows, want.size), want)
+        ix.profile(True)
+        ans = torch.empty(want.size, dtype=torch.int64, device="cuda")
+        ix.search_reads(torch.from_numpy(letters.copy()).cuda(), torch.from_numpy(rows.view(np.int64)).cuda(), ans, want.size)
+        torch.cuda.synchronize()
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert (ix.last_profile()["search_blocks"] < sms) == walks
