@@ -324,9 +324,7 @@ extern "C" void sbwt_index_free(sbwt_index *ix) {
     cudaFree(ix->d_pre);
     cudaFree(ix->d_pre32);
     cudaFree(ix->d_scan);
-    cudaFree(ix->d_node);
-    cudaFree(ix->d_sel);
-    sbwt::free_walk(ix);
+    sbwt::free_stream(ix);
     for (int i = 0; i < sbwt_index::kPipeSlots; i++) {
         ix->ws[i].release();
         if (ix->pipe_stream[i]) cudaStreamDestroy(ix->pipe_stream[i]);

@@ -152,10 +152,12 @@ struct sbwt_index {
     uint32_t *d_pre32 = nullptr;
     bool pre64 = false;
     int compact_pre = -1;  // the compact table: -1 = from SBWT_PRESEARCH_COMPACT, 0 = off, 1 = on
-    // structures of the backward step (stream.cu): node nibbles, select samples
+    // structures of the backward step (stream.cu): node nibbles, select samples, both in stream_mem
+    void *stream_mem = nullptr;
     uint8_t *d_node = nullptr;
     uint32_t *d_sel = nullptr;
-    // structures of the forward walk (WalkView, stream.cuh); walk_q = 0: not there
+    // structures of the forward walk (WalkView, stream.cuh), all in walk_mem; walk_q = 0: not there
+    void *walk_mem = nullptr;
     uint64_t *d_labels = nullptr;
     uint32_t *d_qbits = nullptr, *d_marks = nullptr, *d_path_node = nullptr, *d_node_pos = nullptr;
     ulonglong2 *d_path = nullptr;
@@ -226,7 +228,7 @@ int launch_kmer_list(const SearchArgs &a, uint64_t j0, uint64_t count, uint64_t 
 // stream.cu
 int build_stream(sbwt_index *ix, cudaStream_t s);
 dev::StreamView stream_view(const sbwt_index *ix);
-void free_walk(sbwt_index *ix);
+void free_stream(sbwt_index *ix);
 dev::WalkView walk_view(const sbwt_index *ix);
 
 // packed_runs.cu
