@@ -78,10 +78,11 @@ typedef struct {
  *   graph: an absent stretch is found in a bitmap of the substrings of q
  *   letters, a present k-mer by a search in the sorted labels, and the k-mers
  *   behind it by comparing the read with the path's text.  Serves every
- *   layout of an index within the line layout's size limit, and needs about
- *   17.2 bytes per column and the bitmap (at most 32 MiB up to 4^14 columns),
- *   built on the GPU when the mode is selected.  Lists of single k-mers are
- *   searched through the same structures. */
+ *   layout of an index within the line layout's size limit (on the 32-byte
+ *   lines: poppy and wide-line ranks are read in the other modes), and needs
+ *   about 17.2 bytes per column and the bitmap (at most 32 MiB up to 4^14
+ *   columns), built on the GPU when the mode is selected.  Lists of single
+ *   k-mers are searched through the same structures. */
 #define SBWT_SEARCH_EVERY_KMER 0
 #define SBWT_SEARCH_SKIP_ABSENT 1
 #define SBWT_SEARCH_STREAM 2

@@ -152,7 +152,7 @@ class Index:
         return {"lines_ms": ms[0], "poppy_ms": ms[1], "presearch_ms": ms[2], "backward_ms": ms[3]}
 
     def set_walk_options(self, window=None, blocks_per_sm=None, evict=None, l2_persist=None):
-        """Knobs of the run walk (None: unchanged): window 64/128/256, resident blocks per SM (0: as many
+        """Knobs of the walks (None: unchanged): window 64/128/256, resident blocks per SM (0: as many
         as fit), evict 0 (by table size) / 1 (never) / 2 (always), l2_persist 0/1."""
         keep = 0xFFFFFFFF
         check(lib.sbwt_set_walk_options(self._h, keep if window is None else int(window),
@@ -185,7 +185,7 @@ class Index:
 
     def autotune(self, d_letters, d_row_starts, d_answers, n_kmers, tune_p=False, tune_poppy=False,
                  tune_shapes=False):
-        """Times candidate layouts and run-walk knobs (and p, poppy layouts, per-k-mer kernel shapes on
+        """Times candidate layouts and walk knobs (and p, poppy layouts, per-k-mer kernel shapes on
         request) on a device sample, keeps the fastest; returns the JSON report."""
         n_rows = int(d_row_starts.numel()) - 1
         flags = (2 if tune_p else 0) | (4 if tune_poppy else 0) | (8 if tune_shapes else 0)

@@ -80,11 +80,11 @@ struct KernelShape {
     int kind = SBWT_POPPY;
     int shuffles = 0;
     int mode = SBWT_SEARCH_STREAM;  // batches of reads with the queue-fed form (sbwt_params.search_mode)
-    // knobs of the run walk (batches of reads), set by the autotuner:
+    // knobs of the walks (batches of reads), set by the autotuner:
     u32 window = 128;        // k-mers per window (line layout: 64, 128 or 256)
     u32 blocks_per_sm = 0;   // resident blocks per SM of the persistent grid (0: as many as fit)
     int evict = 0;           // evict-first gathers: 0 = when a table exceeds half of L2, 1 = never, 2 = always
-    int l2_persist = 0;      // the rank lines of the search layout held in the L2 set-aside (l2_window)
+    int l2_persist = 0;      // the rank lines that the search reads held in the L2 set-aside (l2_window)
     int index64 = 0;         // 64-bit k-mer and letter indices even for batches that fit 32 bits
 };
 
